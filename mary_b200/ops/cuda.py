@@ -154,6 +154,19 @@ def _auto_split_k(M: int, N: int, K: int) -> int:
 
 
 declare("mary_gemm_bf16_splitk", "pppiiilllpfiiiplpis")
+declare("mary_gemm_bf16_pair", "pppiiilll" + "iiiiis")
+
+
+def gemm_pair(x, w, bn: int, splits: int = 1, swap: bool = False, glu: str | None = None, f32: bool = False):
+    """The two-SM GEMM with a given tile width and K split (the launchers choose both by themselves)."""
+    _bf16(x), _bf16(w)
+    M, K = x.shape
+    N = w.shape[0] // (2 if glu else 1)
+    out = _empty(M, N, dtype=torch.float32 if f32 else torch.bfloat16, device=x.device)
+    g = 0 if glu is None else {"geglu": 1, "swiglu": 2, "situ": 3}[glu]
+    check(lib().mary_gemm_bf16_pair(_p(x), _p(w), _p(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), g, int(f32), bn, splits, int(swap),
+                                    _stream()), "gemm_bf16_pair")
+    return out
 _SK_WS: dict = {}
 SK_WS_FLOATS = 4 << 20          # 16 MiB of accumulator tiles
 SK_COUNTERS = 8192
@@ -295,9 +308,7 @@ def linear_glu(x, w_gu, act: str = "geglu", limit: float = 0.0, out=None):
         return step_matvec(x, w_gu, mode=act, alpha=limit if act == "clamped" else 1.0, out=out)
     else:
         with static_weights:
-            if M <= 128:
-                return gemm(x, w_gu, out=out, glu=act, limit=limit)
-            y = glu(gemm(x, w_gu), act, limit, out)
+            return gemm(x, w_gu, out=out, glu=act, limit=limit)
     return y if out is None or out is y else out.copy_(y)
 
 
