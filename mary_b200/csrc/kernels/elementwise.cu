@@ -12,33 +12,6 @@ namespace {
 
 constexpr int NT = 256;
 
-__device__ __forceinline__ float block_sum(float v, float* red) {
-  v = warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  float t = (l < (blockDim.x >> 5)) ? red[l] : 0.f;
-  t = warp_sum(t);
-  __syncthreads();
-  return t;
-}
-
-template <typename T> __device__ __forceinline__ float ld(const T* p, int64_t i);
-template <> __device__ __forceinline__ float ld<float>(const float* p, int64_t i) { return p[i]; }
-template <> __device__ __forceinline__ float ld<__nv_bfloat16>(const __nv_bfloat16* p, int64_t i) { return __bfloat162float(p[i]); }
-
-// 8-element vector access helpers (H % 8 == 0, rows 16-byte aligned)
-template <typename T> __device__ __forceinline__ void load8(const T* p, float* f);
-template <> __device__ __forceinline__ void load8<float>(const float* p, float* f) {
-  const float4 a = *(const float4*)p, b = *(const float4*)(p + 4);
-  f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
-}
-template <> __device__ __forceinline__ void load8<__nv_bfloat16>(const __nv_bfloat16* p, float* f) {
-  const uint4 v = *(const uint4*)p;
-  const __nv_bfloat162* h = (const __nv_bfloat162*)&v;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) { float2 t = __bfloat1622float2(h[j]); f[2 * j] = t.x; f[2 * j + 1] = t.y; }
-}
 __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) {
   uint4 v;
   __nv_bfloat162* h = (__nv_bfloat162*)&v;
@@ -47,99 +20,172 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, const float* f) {
   *(uint4*)p = v;
 }
 
+// The norm kernels hold a row in registers: a thread owns CH chunks of 8 neighbouring values (CH 1 up to 4096 values, 3 up to 12288), everything that a
+// row needs is requested before the first sum, and a sum costs one barrier.  Bound: memory for many rows, for one row the chain launch - load - sum -
+// sum - store.  With the row in shared memory, walked by 256 threads, norm_add_norm took 67 us for 8192 rows of 3840 (252 MB) and 4.7 us for one.
+constexpr int MAX_NORM_WARPS = 16;
+
+__device__ __forceinline__ float row_sum(float v, float* red) {
+  v = warp_sum(v);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) red[w] = v;
+  __syncthreads();
+  return warp_sum(l < (int)(blockDim.x >> 5) ? red[l] : 0.f);
+}
+
+template <typename T> struct Raw8;                         // 8 values as they lie in memory
+template <> struct Raw8<float> { float4 a, b; };
+template <> struct Raw8<__nv_bfloat16> { uint4 a; };
+__device__ __forceinline__ void get8(const float* p, Raw8<float>& r) { r.a = *(const float4*)p; r.b = *(const float4*)(p + 4); }
+__device__ __forceinline__ void get8(const __nv_bfloat16* p, Raw8<__nv_bfloat16>& r) { r.a = *(const uint4*)p; }
+__device__ __forceinline__ void widen(const Raw8<float>& r, float* f) { *(float4*)f = r.a; *(float4*)(f + 4) = r.b; }
+__device__ __forceinline__ void widen(const Raw8<__nv_bfloat16>& r, float* f) {
+  const __nv_bfloat162* h = (const __nv_bfloat162*)&r.a;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { float2 t = __bfloat1622float2(h[j]); f[2 * j] = t.x; f[2 * j + 1] = t.y; }
+}
+
 // y = rms(x) * w   (w may be null).  x is bf16 or f32, y bf16.
-template <typename TI>
-__global__ void rmsnorm_kernel(const TI* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                               int H, int64_t ldx, int64_t ldy, float eps) {
+template <typename TI, int CH>
+__global__ void __launch_bounds__(MAX_NORM_WARPS * 32)
+rmsnorm_kernel(const TI* __restrict__ x, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int H, int64_t ldx, int64_t ldy, float eps) {
   pdl_sync();
-  extern __shared__ float row[];
-  __shared__ float red[32];
+  __shared__ float red[MAX_NORM_WARPS];
   const TI* xr = x + (int64_t)blockIdx.x * ldx;
-  float ss = 0.f;
-  for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    float f[8];
-    load8(xr + i, f);
+  Raw8<TI> xv[CH];
+  Raw8<__nv_bfloat16> g[CH];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { row[i + j] = f[j]; ss += f[j] * f[j]; }
+  for (int c = 0; c < CH; ++c) {
+    const int i = (threadIdx.x + c * blockDim.x) * 8;
+    if (i < H) { get8(xr + i, xv[c]); if (w) get8(w + i, g[c]); }
   }
-  const float inv = rsqrtf(block_sum(ss, red) / H + eps);
-  __nv_bfloat16* yr = y + (int64_t)blockIdx.x * ldy;
-  for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    float f[8], g[8];
-    if (w) load8(w + i, g);
+  float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = row[i + j] * inv * (w ? g[j] : 1.f);
-    store8(yr + i, f);
+  for (int c = 0; c < CH; ++c) {
+    if ((threadIdx.x + c * blockDim.x) * 8 < H) {
+      float f[8];
+      widen(xv[c], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
+  }
+  const float inv = rsqrtf(row_sum(ss, red) / H + eps);
+  __nv_bfloat16* yr = y + (int64_t)blockIdx.x * ldy;
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int i = (threadIdx.x + c * blockDim.x) * 8;
+    if (i < H) {
+      float f[8], q[8];
+      widen(xv[c], f);
+      if (w) widen(g[c], q);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * inv * (w ? q[j] : 1.f);
+      store8(yr + i, f);
+    }
   }
 }
 
 // residual += x (one rounding to bf16); y = rms(residual) * w
-template <typename TI>
-__global__ void add_rmsnorm_kernel(const TI* __restrict__ x, __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w,
-                                   __nv_bfloat16* __restrict__ y, int H, float eps) {
+template <typename TI, int CH>
+__global__ void __launch_bounds__(MAX_NORM_WARPS * 32)
+add_rmsnorm_kernel(const TI* __restrict__ x, __nv_bfloat16* __restrict__ res, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y, int H,
+                   float eps) {
   pdl_sync();
-  extern __shared__ float row[];
-  __shared__ float red[32];
+  __shared__ float red[MAX_NORM_WARPS];
   const int64_t o = (int64_t)blockIdx.x * H;
-  float ss = 0.f;
-  for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    float a[8], r[8];
-    load8(x + o + i, a);
-    load8(res + o + i, r);
+  Raw8<TI> xv[CH];
+  Raw8<__nv_bfloat16> rv[CH], g[CH];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) r[j] = __bfloat162float(__float2bfloat16(r[j] + a[j]));
-    store8(res + o + i, r);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { row[i + j] = r[j]; ss += r[j] * r[j]; }
+  for (int c = 0; c < CH; ++c) {
+    const int i = (threadIdx.x + c * blockDim.x) * 8;
+    if (i < H) { get8(x + o + i, xv[c]); get8(res + o + i, rv[c]); get8(w + i, g[c]); }
   }
-  const float inv = rsqrtf(block_sum(ss, red) / H + eps);
-  for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    float f[8], g[8];
-    load8(w + i, g);
+  float r[CH][8];
+  float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = row[i + j] * inv * g[j];
-    store8(y + o + i, f);
+  for (int c = 0; c < CH; ++c) {
+    const int i = (threadIdx.x + c * blockDim.x) * 8;
+    if (i < H) {
+      float a[8];
+      widen(xv[c], a);
+      widen(rv[c], r[c]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { r[c][j] = __bfloat162float(__float2bfloat16(r[c][j] + a[j])); ss += r[c][j] * r[c][j]; }
+      store8(res + o + i, r[c]);
+    }
+  }
+  const float inv = rsqrtf(row_sum(ss, red) / H + eps);
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int i = (threadIdx.x + c * blockDim.x) * 8;
+    if (i < H) {
+      float q[8];
+      widen(g[c], q);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) r[c][j] = r[c][j] * inv * q[j];
+      store8(y + o + i, r[c]);
+    }
   }
 }
 
 // Gemma sandwich step: h = (h + rms(a) * w_post) * scalar ; x = rms(h) * w_next (skipped when w_next is null)
-template <typename TI>
-__global__ void norm_add_norm_kernel(const TI* __restrict__ a, const __nv_bfloat16* __restrict__ w_post, __nv_bfloat16* __restrict__ h,
-                                     const __nv_bfloat16* __restrict__ w_next, __nv_bfloat16* __restrict__ xo, int H, float eps, float scalar) {
+template <typename TI, int CH>
+__global__ void __launch_bounds__(MAX_NORM_WARPS * 32)
+norm_add_norm_kernel(const TI* __restrict__ a, const __nv_bfloat16* __restrict__ w_post, __nv_bfloat16* __restrict__ h,
+                     const __nv_bfloat16* __restrict__ w_next, __nv_bfloat16* __restrict__ xo, int H, float eps, float scalar) {
   pdl_sync();
-  extern __shared__ float row[];
-  __shared__ float red[32];
+  __shared__ float red[2][MAX_NORM_WARPS];
   const int64_t o = (int64_t)blockIdx.x * H;
-  float ss = 0.f;
-  for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    float f[8];
-    load8(a + o + i, f);
+  Raw8<TI> av[CH];
+  Raw8<__nv_bfloat16> hv[CH], gp[CH], gn[CH];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) { row[i + j] = f[j]; ss += f[j] * f[j]; }
+  for (int c = 0; c < CH; ++c) {
+    const int i = (threadIdx.x + c * blockDim.x) * 8;
+    if (i < H) { get8(a + o + i, av[c]); get8(h + o + i, hv[c]); get8(w_post + i, gp[c]); if (w_next) get8(w_next + i, gn[c]); }
   }
-  const float inv = rsqrtf(block_sum(ss, red) / H + eps);
-  float ss2 = 0.f;
-  for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    float g[8], r[8];
-    load8(w_post + i, g);
-    load8(h + o + i, r);
+  float ss = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      // the normed branch output is rounded to bf16 like the unfused op sequence would
-      const float n = __bfloat162float(__float2bfloat16(row[i + j] * inv * g[j]));
-      r[j] = __bfloat162float(__float2bfloat16((r[j] + n) * scalar));
-      row[i + j] = r[j]; ss2 += r[j] * r[j];
+  for (int c = 0; c < CH; ++c) {
+    if ((threadIdx.x + c * blockDim.x) * 8 < H) {
+      float f[8];
+      widen(av[c], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
     }
-    store8(h + o + i, r);
+  }
+  const float inv = rsqrtf(row_sum(ss, red[0]) / H + eps);
+  float r[CH][8];
+  float ss2 = 0.f;
+#pragma unroll
+  for (int c = 0; c < CH; ++c) {
+    const int i = (threadIdx.x + c * blockDim.x) * 8;
+    if (i < H) {
+      float f[8], g[8];
+      widen(av[c], f);
+      widen(gp[c], g);
+      widen(hv[c], r[c]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        // the normed branch output is rounded to bf16 like the unfused op sequence would
+        const float n = __bfloat162float(__float2bfloat16(f[j] * inv * g[j]));
+        r[c][j] = __bfloat162float(__float2bfloat16((r[c][j] + n) * scalar));
+        ss2 += r[c][j] * r[c][j];
+      }
+      store8(h + o + i, r[c]);
+    }
   }
   if (w_next == nullptr) return;
-  const float inv2 = rsqrtf(block_sum(ss2, red) / H + eps);
-  for (int i = threadIdx.x * 8; i < H; i += blockDim.x * 8) {
-    float f[8], g[8];
-    load8(w_next + i, g);
+  const float inv2 = rsqrtf(row_sum(ss2, red[1]) / H + eps);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = row[i + j] * inv2 * g[j];
-    store8(xo + o + i, f);
+  for (int c = 0; c < CH; ++c) {
+    const int i = (threadIdx.x + c * blockDim.x) * 8;
+    if (i < H) {
+      float g[8];
+      widen(gn[c], g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) r[c][j] = r[c][j] * inv2 * g[j];
+      store8(xo + o + i, r[c]);
+    }
   }
 }
 
@@ -181,6 +227,84 @@ __global__ void embed_kernel(const int* __restrict__ ids, const __nv_bfloat16* _
       for (int j = 0; j < 4; ++j) { float2 f = __bfloat1622float2(p[j]); p[j] = __floats2bfloat162_rn(f.x * scale, f.y * scale); }
     }
     *(uint4*)(dst + i) = v;
+  }
+}
+
+// The same as the kernel below for heads of 64 * E values whose rows are aligned: a lane owns E neighbouring pairs (i, i + D / 2), so a head is two
+// vector loads and stores per lane, and a warp takes HPW heads of one token, all requested before the first is used, with one set of angles.
+// One head per warp and 2-byte accesses took 182 us for 8192 tokens of 32 heads of 256 (268 MB).
+template <int E> struct Pairs;
+template <> struct Pairs<1> { using T = uint16_t; };
+template <> struct Pairs<2> { using T = uint32_t; };
+template <> struct Pairs<4> { using T = uint2; };
+template <> struct Pairs<8> { using T = uint4; };
+
+template <int E, int HPW>
+__global__ void __launch_bounds__(256)
+qk_norm_rope_rows_kernel(const __nv_bfloat16* __restrict__ qkv, int n_q, int n_kv, const __nv_bfloat16* __restrict__ q_norm,
+                         const __nv_bfloat16* __restrict__ k_norm, int v_norm, const float* __restrict__ inv_freq, const int* __restrict__ positions,
+                         const int64_t* __restrict__ slots, __nv_bfloat16* __restrict__ qo, __nv_bfloat16* __restrict__ kc, __nv_bfloat16* __restrict__ vc,
+                         float eps, int T, int64_t n_slots, int* __restrict__ status) {
+  pdl_sync();
+  constexpr int HALF = 32 * E, D = 2 * HALF;
+  using V = typename Pairs<E>::T;
+  union Piece { V v; __nv_bfloat16 e[E]; };
+  const int heads = n_q + 2 * n_kv, groups = (heads + HPW - 1) / HPW;
+  const int64_t gw = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (gw >= (int64_t)T * groups) return;
+  const int t = (int)(gw / groups), h0 = (int)(gw % groups) * HPW, lane = threadIdx.x & 31;
+  const __nv_bfloat16* src = qkv + ((int64_t)t * heads + h0) * D + lane * E;
+  Piece a[HPW], b[HPW];
+#pragma unroll
+  for (int k = 0; k < HPW; ++k) {
+    if (h0 + k < heads) { a[k].v = *(const V*)(src + k * D); b[k].v = *(const V*)(src + k * D + HALF); }
+  }
+  const float pos = (float)positions[t];
+  const int64_t slot = n_kv > 0 ? slots[t] : 0;
+  const bool slot_ok = n_slots <= 0 || (slot >= 0 && slot < n_slots);
+  float sn[E], cs[E];
+  const bool turn = inv_freq != nullptr && h0 < n_q + n_kv;
+  if (turn) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) sincosf(pos * inv_freq[lane * E + e], &sn[e], &cs[e]);
+  }
+#pragma unroll
+  for (int k = 0; k < HPW; ++k) {
+    const int hh = h0 + k;
+    if (hh >= heads) break;
+    const bool is_q = hh < n_q, is_k = !is_q && hh < n_q + n_kv;
+    if (!is_q && !slot_ok) { if (lane == 0) atomicCAS(status, 0, (int)MARY_ERR_BOUNDS); continue; }       // outside the cache: recorded, not written
+    const __nv_bfloat16* gain = is_q ? q_norm : (is_k ? k_norm : nullptr);
+    const bool do_norm = is_q ? (q_norm != nullptr) : (is_k ? (k_norm != nullptr) : (v_norm != 0));
+    float x1[E], x2[E], ss = 0.f;
+#pragma unroll
+    for (int e = 0; e < E; ++e) {
+      x1[e] = __bfloat162float(a[k].e[e]); x2[e] = __bfloat162float(b[k].e[e]);
+      ss += x1[e] * x1[e] + x2[e] * x2[e];
+    }
+    if (do_norm) {
+      const float inv = rsqrtf(warp_sum(ss) / D + eps);
+      Piece g1, g2;
+      if (gain) { g1.v = *(const V*)(gain + lane * E); g2.v = *(const V*)(gain + HALF + lane * E); }
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        // round the normed value to bf16 first, as the unfused sequence (norm kernel then rope kernel) does
+        x1[e] = __bfloat162float(__float2bfloat16(x1[e] * inv * (gain ? __bfloat162float(g1.e[e]) : 1.f)));
+        x2[e] = __bfloat162float(__float2bfloat16(x2[e] * inv * (gain ? __bfloat162float(g2.e[e]) : 1.f)));
+      }
+    }
+    if (turn && (is_q || is_k)) {
+#pragma unroll
+      for (int e = 0; e < E; ++e) {
+        const float ra = x1[e] * cs[e] - x2[e] * sn[e], rb = x1[e] * sn[e] + x2[e] * cs[e];
+        x1[e] = ra; x2[e] = rb;
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < E; ++e) { a[k].e[e] = __float2bfloat16(x1[e]); b[k].e[e] = __float2bfloat16(x2[e]); }
+    __nv_bfloat16* dst = is_q ? qo + ((int64_t)t * n_q + hh) * D : (is_k ? kc + (slot * n_kv + (hh - n_q)) * D : vc + (slot * n_kv + (hh - n_q - n_kv)) * D);
+    *(V*)(dst + lane * E) = a[k].v;
+    *(V*)(dst + HALF + lane * E) = b[k].v;
   }
 }
 
@@ -272,23 +396,33 @@ __global__ void short_conv_kernel(const __nv_bfloat16* __restrict__ x, const flo
 
 }  // namespace
 
+// Threads of a norm kernel whose threads own `ch` chunks of 8 values each
+static int norm_threads(int H, int ch) { return ((H / 8 + ch - 1) / ch + 31) / 32 * 32; }
+static int norm_chunks(int H) { return (H / 8 + MAX_NORM_WARPS * 32 - 1) / (MAX_NORM_WARPS * 32); }
+#define MARY_NORM(kernel_, TI_, T_, H_, s_, ...)                                                                    \
+  do {                                                                                                              \
+    switch (norm_chunks(H_)) {                                                                                      \
+      case 1: MARY_LAUNCH((kernel_<TI_, 1>), T_, norm_threads(H_, 1), 0, s_, __VA_ARGS__); break;                    \
+      case 2: MARY_LAUNCH((kernel_<TI_, 2>), T_, norm_threads(H_, 2), 0, s_, __VA_ARGS__); break;                    \
+      default: MARY_LAUNCH((kernel_<TI_, 3>), T_, norm_threads(H_, 3), 0, s_, __VA_ARGS__);                          \
+    }                                                                                                               \
+  } while (0)
+
 MARY_API int mary_rmsnorm(const void* x, int x_is_f32, const void* w, void* y, int T, int H, int64_t ldx, int64_t ldy, float eps,
                           cudaStream_t s) {
   if (T <= 0) return MARY_OK;
-  size_t sm = (size_t)H * 4;
-  if (sm > 48 * 1024 || (H & 7) || (ldx & 7) || (ldy & 7)) return MARY_ERR_BAD_ARG;
-  if (x_is_f32) MARY_LAUNCH((rmsnorm_kernel<float>), T, NT, sm, s, (const float*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, H, ldx, ldy, eps);
-  else MARY_LAUNCH((rmsnorm_kernel<__nv_bfloat16>), T, NT, sm, s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, H, ldx, ldy, eps);
+  if (H <= 0 || H > 12288 || (H & 7) || (ldx & 7) || (ldy & 7)) return MARY_ERR_BAD_ARG;
+  if (x_is_f32) MARY_NORM(rmsnorm_kernel, float, T, H, s, (const float*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, H, ldx, ldy, eps);
+  else MARY_NORM(rmsnorm_kernel, __nv_bfloat16, T, H, s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, H, ldx, ldy, eps);
   MARY_CHECK_LAUNCH();
   return MARY_OK;
 }
 
 MARY_API int mary_add_rmsnorm(const void* x, int x_is_f32, void* res, const void* w, void* y, int T, int H, float eps, cudaStream_t s) {
   if (T <= 0) return MARY_OK;
-  size_t sm = (size_t)H * 4;
-  if (sm > 48 * 1024 || (H & 7)) return MARY_ERR_BAD_ARG;
-  if (x_is_f32) MARY_LAUNCH((add_rmsnorm_kernel<float>), T, NT, sm, s, (const float*)x, (__nv_bfloat16*)res, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, H, eps);
-  else MARY_LAUNCH((add_rmsnorm_kernel<__nv_bfloat16>), T, NT, sm, s, (const __nv_bfloat16*)x, (__nv_bfloat16*)res, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, H, eps);
+  if (H <= 0 || H > 12288 || (H & 7)) return MARY_ERR_BAD_ARG;
+  if (x_is_f32) MARY_NORM(add_rmsnorm_kernel, float, T, H, s, (const float*)x, (__nv_bfloat16*)res, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, H, eps);
+  else MARY_NORM(add_rmsnorm_kernel, __nv_bfloat16, T, H, s, (const __nv_bfloat16*)x, (__nv_bfloat16*)res, (const __nv_bfloat16*)w, (__nv_bfloat16*)y, H, eps);
   MARY_CHECK_LAUNCH();
   return MARY_OK;
 }
@@ -296,10 +430,9 @@ MARY_API int mary_add_rmsnorm(const void* x, int x_is_f32, void* res, const void
 MARY_API int mary_norm_add_norm(const void* a, int a_is_f32, const void* w_post, void* h, const void* w_next, void* xo, int T, int H,
                                 float eps, float scalar, cudaStream_t s) {
   if (T <= 0) return MARY_OK;
-  size_t sm = (size_t)H * 4;
-  if (sm > 48 * 1024 || (H & 7)) return MARY_ERR_BAD_ARG;
-  if (a_is_f32) MARY_LAUNCH((norm_add_norm_kernel<float>), T, NT, sm, s, (const float*)a, (const __nv_bfloat16*)w_post, (__nv_bfloat16*)h, (const __nv_bfloat16*)w_next, (__nv_bfloat16*)xo, H, eps, scalar);
-  else MARY_LAUNCH((norm_add_norm_kernel<__nv_bfloat16>), T, NT, sm, s, (const __nv_bfloat16*)a, (const __nv_bfloat16*)w_post, (__nv_bfloat16*)h, (const __nv_bfloat16*)w_next, (__nv_bfloat16*)xo, H, eps, scalar);
+  if (H <= 0 || H > 12288 || (H & 7)) return MARY_ERR_BAD_ARG;
+  if (a_is_f32) MARY_NORM(norm_add_norm_kernel, float, T, H, s, (const float*)a, (const __nv_bfloat16*)w_post, (__nv_bfloat16*)h, (const __nv_bfloat16*)w_next, (__nv_bfloat16*)xo, H, eps, scalar);
+  else MARY_NORM(norm_add_norm_kernel, __nv_bfloat16, T, H, s, (const __nv_bfloat16*)a, (const __nv_bfloat16*)w_post, (__nv_bfloat16*)h, (const __nv_bfloat16*)w_next, (__nv_bfloat16*)xo, H, eps, scalar);
   MARY_CHECK_LAUNCH();
   return MARY_OK;
 }
@@ -329,7 +462,25 @@ MARY_API int mary_qk_norm_rope_append(const void* qkv, int n_q, int n_kv, int D,
                                       float eps, int T, int64_t n_slots, cudaStream_t s) {
   if (T <= 0) return MARY_OK;
   if (D > 512 || (D & 1)) return MARY_ERR_BAD_ARG;
-  const int64_t warps = (int64_t)T * (n_q + 2 * n_kv);
+  const int heads = n_q + 2 * n_kv;
+  const uintptr_t at = (uintptr_t)qkv | (uintptr_t)qo | (uintptr_t)q_norm | (uintptr_t)k_norm | (n_kv ? (uintptr_t)kc | (uintptr_t)vc : 0);
+  const int E = D / 64;
+  if (D % 64 == 0 && (E == 1 || E == 2 || E == 4 || E == 8) && at % (2 * E) == 0) {
+    // four heads per warp once that still gives every SM a dozen warps; before that the chain of one head is what counts
+    const bool wide = (int64_t)T * ((heads + 3) / 4) >= (int64_t)mary_num_sms() * 12;
+    const int64_t w = (int64_t)T * (wide ? (heads + 3) / 4 : heads);
+#define MARY_QK(E_, HPW_) MARY_LAUNCH((qk_norm_rope_rows_kernel<E_, HPW_>), (int)((w + 7) / 8), 256, 0, s, (const __nv_bfloat16*)qkv, n_q, n_kv, \
+    (const __nv_bfloat16*)q_norm, (const __nv_bfloat16*)k_norm, v_norm, inv_freq, positions, slots, (__nv_bfloat16*)qo, (__nv_bfloat16*)kc,       \
+    (__nv_bfloat16*)vc, eps, T, n_slots, mary_status_ptr())
+    if (E == 1) { if (wide) MARY_QK(1, 4); else MARY_QK(1, 1); }
+    else if (E == 2) { if (wide) MARY_QK(2, 4); else MARY_QK(2, 1); }
+    else if (E == 4) { if (wide) MARY_QK(4, 4); else MARY_QK(4, 1); }
+    else { if (wide) MARY_QK(8, 4); else MARY_QK(8, 1); }
+#undef MARY_QK
+    MARY_CHECK_LAUNCH();
+    return MARY_OK;
+  }
+  const int64_t warps = (int64_t)T * heads;
   const int wpb = 8;
   MARY_LAUNCH(qk_norm_rope_append_kernel, (int)((warps + wpb - 1) / wpb), wpb * 32, 0, s, 
       (const __nv_bfloat16*)qkv, n_q, n_kv, D, (const __nv_bfloat16*)q_norm, (const __nv_bfloat16*)k_norm, v_norm, inv_freq, positions,
