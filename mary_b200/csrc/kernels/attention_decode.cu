@@ -12,7 +12,6 @@
 #include "attention_form.cuh"
 #include "common.cuh"
 #include "host_utils.h"
-#include <type_traits>
 
 using namespace mary;
 
@@ -31,9 +30,6 @@ struct DecParams {
   int Hq, Hkv, G, RQ, nsplit, window;
   float scale, softcap;
   int64_t out_ld;              // elements between the output rows of two tokens
-  // 8-bit cache: kc / vc hold one unsigned code per element and the strides count codes; k_sz / v_sz hold (scale, zero) of every
-  // (slot, kv head) as two floats, slot-major; element = code * scale + zero
-  const float* k_sz; const float* v_sz;
   const float* bias;           // [Hq][window] by distance, added to the scaled score; or null
   const __nv_bfloat16* gate;   // rows of gate_ld elements, head h at h * D: the output times its logistic function; or null
   int64_t gate_ld;
@@ -64,18 +60,6 @@ __device__ __forceinline__ void unpack(const typename Vec<E>::T& v, float* f) {
   const __nv_bfloat162* h = (const __nv_bfloat162*)&v;
 #pragma unroll
   for (int j = 0; j < E / 2; ++j) { float2 t = __bfloat1622float2(h[j]); f[2 * j] = t.x; f[2 * j + 1] = t.y; }
-}
-
-template <int E> struct QVec;                      // E 8-bit codes per lane
-template <> struct QVec<2> { using T = uint16_t; };
-template <> struct QVec<4> { using T = uint32_t; };
-template <> struct QVec<8> { using T = uint2; };
-
-template <int E>
-__device__ __forceinline__ void unpack_q8(const typename QVec<E>::T& v, float sc, float zero, float* f) {
-  const uint8_t* b = (const uint8_t*)&v;
-#pragma unroll
-  for (int j = 0; j < E; ++j) f[j] = fmaf((float)b[j], sc, zero);
 }
 
 // Sums V values (a power of two, at most 32) over the 32 lanes and leaves ALL V totals in every lane.  Instead of one
@@ -116,7 +100,7 @@ __device__ __forceinline__ void warp_sum_vec(float* v, float* other, int lane, f
 // FORM: chunks, the sink and the query temperature of p.f are honoured and the cap is exact.  MAPS = 2: key and query rows are
 // [map 0 | map 1] of D values each, a half warp each; the partials of row r and map m are row 2 r + m of the scratch, and only partials
 // are written.
-template <int D, int DV, int RMAX, bool Q8, int MAPS, bool FORM>
+template <int D, int DV, int RMAX, int MAPS, bool FORM>
 __global__ void __launch_bounds__(WARPS * 32)
 attn_decode_kernel(const DecParams p) {
   pdl_sync();
@@ -126,8 +110,7 @@ attn_decode_kernel(const DecParams p) {
   constexpr int RT = RMAX * MAPS;
   static_assert(RT <= MAXR, "rows of the scratch");
   using V = typename Vec<E>::T;
-  using KV = typename std::conditional<Q8, typename QVec<E>::T, V>::type;
-  using VV = typename std::conditional<Q8, typename QVec<EV>::T, typename Vec<EV>::T>::type;
+  using VV = typename Vec<EV>::T;
   __shared__ float red_o[WARPS][RT][DV];
   __shared__ float red_ml[WARPS][RT][2];
   const int nb = blockIdx.x, kvh = blockIdx.y, split = blockIdx.z;
@@ -169,26 +152,15 @@ attn_decode_kernel(const DecParams p) {
   const int* pt = p.page_table + (int64_t)seq * p.max_pages;
 
   for (int kb = s_lo + warp * KG; kb < s_hi; kb += WARPS * KG) {
-    KV kv[KG];
+    V kv[KG];
     VV vv[KG];
-    float2 ksz[KG], vsz[KG];
 #pragma unroll
     for (int j = 0; j < KG; ++j) {
       const int kp = min(kb + j, s_hi - 1);          // clamped: masked below
       const int page = pt[kp / p.page_size];
       const int64_t tok = kp % p.page_size;
-      if constexpr (Q8) {
-        const uint8_t* kq = (const uint8_t*)p.kc;
-        const uint8_t* vq = (const uint8_t*)p.vc;
-        kv[j] = *(const KV*)(kq + (int64_t)page * p.k_page + tok * p.k_tok + (int64_t)kvh * D + lane * E);
-        vv[j] = *(const VV*)(vq + (int64_t)page * p.v_page + tok * p.v_tok + (int64_t)kvh * DV + lane * EV);
-        const int64_t slot = ((int64_t)page * p.page_size + tok) * p.Hkv + kvh;
-        ksz[j] = *(const float2*)(p.k_sz + slot * 2);
-        vsz[j] = *(const float2*)(p.v_sz + slot * 2);
-      } else {
-        kv[j] = *(const KV*)(p.kc + (int64_t)page * p.k_page + tok * p.k_tok + (int64_t)kvh * DR + lane * E);
-        vv[j] = *(const VV*)(p.vc + (int64_t)page * p.v_page + tok * p.v_tok + (int64_t)kvh * DV + lane * EV);
-      }
+      kv[j] = *(const V*)(p.kc + (int64_t)page * p.k_page + tok * p.k_tok + (int64_t)kvh * DR + lane * E);
+      vv[j] = *(const VV*)(p.vc + (int64_t)page * p.v_page + tok * p.v_tok + (int64_t)kvh * DV + lane * EV);
     }
     constexpr int LW = 32 / MAPS;                       // lanes that share a dot product
     constexpr int NV = KG * RMAX, NB = (NV + LW - 1) / LW;
@@ -206,8 +178,7 @@ attn_decode_kernel(const DecParams p) {
 #pragma unroll
     for (int j = 0; j < KG; ++j) {
       float kf[E];
-      if constexpr (Q8) unpack_q8<E>(kv[j], ksz[j].x, ksz[j].y, kf);
-      else unpack<E>(kv[j], kf);
+      unpack<E>(kv[j], kf);
 #pragma unroll
       for (int r = 0; r < RMAX; ++r) {
         float a = 0.f;
@@ -256,8 +227,7 @@ attn_decode_kernel(const DecParams p) {
             const float pj = (sv[j] == -INFINITY) ? 0.f : __expf(sv[j] - mx);
             l[r] += pj;
             float vf[EV];
-            if constexpr (Q8) unpack_q8<EV>(vv[j], vsz[j].x, vsz[j].y, vf);
-            else unpack<EV>(vv[j], vf);
+            unpack<EV>(vv[j], vf);
 #pragma unroll
             for (int e = 0; e < EV; ++e) o[r][e] += pj * vf[e];
           }
@@ -370,12 +340,10 @@ __global__ void __launch_bounds__(256) attn_decode_difference_kernel(const DecPa
 template <int D, int RMAX>
 int launch(const DecParams& p, int NB, bool form, cudaStream_t s) {
   const dim3 grid(NB, p.Hkv, p.nsplit);
-  if (p.k_sz) {
-    MARY_LAUNCH((attn_decode_kernel<D, D, RMAX, true, 1, false>), grid, WARPS * 32, 0, s, p);
-  } else if (form) {
-    MARY_LAUNCH((attn_decode_kernel<D, D, RMAX, false, 1, true>), grid, WARPS * 32, 0, s, p);
+  if (form) {
+    MARY_LAUNCH((attn_decode_kernel<D, D, RMAX, 1, true>), grid, WARPS * 32, 0, s, p);
   } else {
-    MARY_LAUNCH((attn_decode_kernel<D, D, RMAX, false, 1, false>), grid, WARPS * 32, 0, s, p);
+    MARY_LAUNCH((attn_decode_kernel<D, D, RMAX, 1, false>), grid, WARPS * 32, 0, s, p);
   }
   MARY_CHECK_LAUNCH();
   if (p.nsplit > 1) {
@@ -387,7 +355,7 @@ int launch(const DecParams& p, int NB, bool form, cudaStream_t s) {
 
 template <int D, int DV, int RMAX>
 int launch_maps(const DecParams& p, int NB, cudaStream_t s) {
-  MARY_LAUNCH((attn_decode_kernel<D, DV, RMAX, false, 2, true>), dim3(NB, p.Hkv, p.nsplit), WARPS * 32, 0, s, p);
+  MARY_LAUNCH((attn_decode_kernel<D, DV, RMAX, 2, true>), dim3(NB, p.Hkv, p.nsplit), WARPS * 32, 0, s, p);
   MARY_CHECK_LAUNCH();
   MARY_LAUNCH((attn_decode_difference_kernel<DV>), dim3(NB, p.Hkv), 256, 0, s, p);
   MARY_CHECK_LAUNCH();
@@ -398,7 +366,7 @@ int launch_maps(const DecParams& p, int NB, cudaStream_t s) {
 
 // Same contract as mary_paged_attention with DK == DV == D in {64, 128, 256} and RQ * (Hq / Hkv) <= 8 (<= 4 for D = 256).
 // Scratch (nsplit > 1): mary_paged_attention_scratch_floats(NB, Hkv, nsplit, D).
-static int decode_run(const void* q, const void* kc, const void* vc, const float* k_sz, const float* v_sz, void* out, const int* page_table,
+static int decode_run(const void* q, const void* kc, const void* vc, void* out, const int* page_table,
                       const int* kv_len, const int* q_start, const int* blk_seq, const int* blk_q0, int NB,
                       int max_pages, int page_size, int64_t k_tok, int64_t k_page, int64_t v_tok, int64_t v_page,
                       int Hq, int Hkv, int D, int RQ, int nsplit, int window, float scale, float softcap,
@@ -409,7 +377,6 @@ static int decode_run(const void* q, const void* kc, const void* vc, const float
   if (bias && window < 1) return MARY_ERR_BAD_ARG;
   DecParams p;
   p.bias = bias; p.gate = (const __nv_bfloat16*)gate; p.gate_ld = gate_ld;
-  p.k_sz = k_sz; p.v_sz = v_sz;
   p.q = (const __nv_bfloat16*)q; p.kc = (const __nv_bfloat16*)kc; p.vc = (const __nv_bfloat16*)vc; p.out = (__nv_bfloat16*)out;
   p.page_table = page_table; p.kv_len = kv_len; p.q_start = q_start; p.blk_seq = blk_seq; p.blk_q0 = blk_q0;
   p.max_pages = max_pages; p.page_size = page_size; p.k_tok = k_tok; p.k_page = k_page; p.v_tok = v_tok; p.v_page = v_page;
@@ -448,21 +415,8 @@ MARY_API int mary_paged_attention_decode(const void* q, const void* kc, const vo
                                          int Hq, int Hkv, int D, int RQ, int nsplit, int window, float scale, float softcap,
                                          float* scratch, int64_t out_ld, const float* bias, const void* gate, int64_t gate_ld,
                                          const MaryAttnForm* form, int DV, cudaStream_t s) {
-  return decode_run(q, kc, vc, nullptr, nullptr, out, page_table, kv_len, q_start, blk_seq, blk_q0, NB, max_pages, page_size, k_tok, k_page,
+  return decode_run(q, kc, vc, out, page_table, kv_len, q_start, blk_seq, blk_q0, NB, max_pages, page_size, k_tok, k_page,
                     v_tok, v_page, Hq, Hkv, D, RQ, nsplit, window, scale, softcap, scratch, s, out_ld, bias, gate, gate_ld, form, DV);
-}
-
-// The same over an 8-bit cache: kc / vc are code pages [pages, page, Hkv, D] of unsigned bytes (strides in bytes), k_sz / v_sz the
-// (scale, zero) pairs [pages * page, Hkv, 2] f32 written by mary_kv_quant_append.  The cache rows are dequantised in registers
-// (one fused multiply-add per element), so the kernel streams half the bytes of the bf16 cache.
-MARY_API int mary_paged_attention_decode_q8(const void* q, const void* kc, const void* vc, const float* k_sz, const float* v_sz, void* out,
-                                            const int* page_table, const int* kv_len, const int* q_start, const int* blk_seq,
-                                            const int* blk_q0, int NB, int max_pages, int page_size, int64_t k_tok, int64_t k_page,
-                                            int64_t v_tok, int64_t v_page, int Hq, int Hkv, int D, int RQ, int nsplit, int window,
-                                            float scale, float softcap, float* scratch, cudaStream_t s) {
-  if (!k_sz || !v_sz) return MARY_ERR_BAD_ARG;
-  return decode_run(q, kc, vc, k_sz, v_sz, out, page_table, kv_len, q_start, blk_seq, blk_q0, NB, max_pages, page_size, k_tok, k_page,
-                    v_tok, v_page, Hq, Hkv, D, RQ, nsplit, window, scale, softcap, scratch, s);
 }
 
 namespace {

@@ -102,7 +102,7 @@ def paged_attention(q, kcache, vcache, meta, scale, window=0, softcap=0.0, rel_b
     With an 8-bit cache, decode-shaped batches run the dequantising kernel; everything else dequantises the pages of the batch."""
     if _is_q8(kcache):
         if _cuda(q) and rel_bias is None and _k().decode_q8_supported(q, kcache, meta):
-            return _k().paged_attention_decode_q8(q, kcache, vcache, meta, scale, window, softcap)
+            return _k().attention_stream(q, kcache, vcache, meta, scale, window, softcap)
         import dataclasses
         need = (meta.kv_len.long() + meta.page_size - 1) // meta.page_size
         cols = torch.arange(meta.page_table.shape[1], device=need.device)[None]

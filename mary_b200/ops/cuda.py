@@ -5,8 +5,10 @@ graphs like any other stream work.  Every wrapper checks the launcher's return c
 from __future__ import annotations
 
 import ctypes
+import functools
 import math
 
+import numpy as np
 import torch
 
 from .. import _native
@@ -474,7 +476,6 @@ def _paged_attention_decode(q, kcache, vcache, meta, scale, window, softcap, nsp
     return out
 
 
-declare("mary_paged_attention_decode_q8", "pppppp" + "ppppp" + "iii" + "llll" + "iiiiii" + "ffps")
 declare("mary_kv_quant_append", "plppp" + "iiils")
 
 
@@ -493,27 +494,75 @@ def decode_q8_supported(q, kcache, meta) -> bool:
             and Hq // Hkv <= (4 if D == 256 else 8) and meta.max_q_len <= 8)
 
 
-def paged_attention_decode_q8(q, kcache, vcache, meta, scale, window=0, softcap=0.0, nsplit=None):
-    """The decode kernel over an 8-bit cache (``runtime.kv_cache.Q8Pages``): rows are dequantised in registers."""
+declare("mary_attention_stream", "ppppppppppp" + "iii" + "llllll" + "iiiiiii" + "ffs")
+
+
+def attention_stream_rows(q, kcache, meta) -> int:
+    """Query tokens per block of the streaming decode kernel, or 0 where it does not take the shape."""
+    D, G = q.shape[2], q.shape[1] // kcache.shape[2]
+    cap = 4 if D == 256 else 8
+    return 0 if D not in (64, 128, 256) or G > cap or q.shape[1] % kcache.shape[2] else max(1, min(cap // G, meta.max_q_len))
+
+
+@functools.lru_cache(maxsize=1024)
+def stream_split(units: int, span: int, sms: int = 148):
+    """``(splits of the key range, warps per CTA, estimated us)`` of the streaming decode kernel for ``units`` (query block, kv head) pairs of ``span``
+    keys: waves of CTAs x (4 us + keys of a CTA x time per key).  A lone warp needs 141 ns per key (eight keys take one chain of load, sum over the lanes,
+    exponential, weighted sum), an SM gets through one key per 25 ns, and the rings let an SM hold three CTAs of 4 warps or one of 8; clusters of 4
+    and 8 CTAs leave 12 and 36 SMs out.  Measured (us) for 256 units of 1024 keys of 256: 1 / 8 56, 1 / 4 57, 4 / 4 67, 2 / 4 78; for 64 units of 2000: 2 / 8
+    30, 4 / 4 33, 2 / 4 40, 1 / 8 50; for 8 of 777: 8 / 8 8, 8 / 4 9, 4 / 8 10, 1 / 4 30."""
+    best = None
+    for nsplit, usable in ((1, sms), (2, sms), (4, sms - 12), (8, sms - 36)):
+        if nsplit > 1 and span < 32 * nsplit:
+            break
+        for warps, fit in ((4, 3), (8, 1)):
+            ctas = units * nsplit
+            waves = -(-ctas // max(1, fit * usable))
+            resident = min(fit, -(-ctas // sms))
+            t = waves * (4.0 + -(-span // nsplit) * max(0.141 / warps, 0.025 * resident))
+            if best is None or t < best[2]:
+                best = (nsplit, warps, t)
+    return best
+
+
+def _stream_wins(q, kcache, vcache, meta, window) -> bool:
+    """Whether the streaming kernel is the faster one for a bf16 batch that the tensor-core kernel takes as well: heads of 256 with at most two rows per kv
+    head (more rows cost it products that the tensor core has to spare: 80 against 54 us at four), unless a few long sequences leave its clusters
+    of 8 CTAs behind (one sequence of 16000: 52 against 37 us).  The tensor-core kernel takes about 10 us + its bytes at 5.3 TB/s."""
+    rq = attention_stream_rows(q, kcache, meta)
+    Hkv = kcache.shape[2]
+    if not rq or q.shape[2] != 256 or rq * (q.shape[1] // Hkv) > 2 or meta.kv_lens_host is None or meta.max_q_len > 8:
+        return False
+    if any((t.data_ptr() | t.stride(0) * 2 | t.stride(1) * 2) % 16 or t.stride(2) != 256 or t.stride(3) != 1 for t in (kcache, vcache)):
+        return False
+    key = ("stream", window, Hkv, rq)
+    memo = meta.__dict__.setdefault("_cache", {})
+    if key not in memo:
+        keys = int(np.minimum(meta.kv_lens_host, window + rq).sum() if window > 0 else meta.kv_lens_host.sum())
+        span = meta.max_kv_len if window <= 0 else min(meta.max_kv_len, window + rq)
+        blocks = sum(-(-n // rq) for n in meta.q_lens_host.tolist())
+        memo[key] = stream_split(blocks * Hkv, span, lib().mary_sm_count())[2] <= 10.0 + keys * Hkv * 1024 / 5.3e6
+    return memo[key]
+
+
+def attention_stream(q, kcache, vcache, meta, scale, window=0, softcap=0.0, nsplit=None, warps=None):
+    """Decode-shaped batches with few rows per kv head (``csrc/kernels/attention_stream.cu``) over a bf16 cache or ``Q8Pages``."""
     T, Hq, D = q.shape
     Hkv = kcache.shape[2]
-    G = Hq // Hkv
-    cap = 4 if D == 256 else 8
-    rq = max(1, min(cap // G, meta.max_q_len))
+    q8 = not isinstance(kcache, torch.Tensor)
+    kc, vc = (kcache.codes, vcache.codes) if q8 else (kcache, vcache)
+    assert kc.stride(3) == 1 and kc.stride(2) == D and vc.stride(3) == 1 and vc.stride(2) == D and kc.shape[3] == D and vc.shape[3] == D
+    rq = attention_stream_rows(q, kcache, meta)
     blk_seq, blk_q0, NB = _q_blocks(meta, rq)
     if nsplit is None:
-        want = max(1, DECODE_TARGET_CTAS // max(1, NB * Hkv))
         span = meta.max_kv_len if window <= 0 else min(meta.max_kv_len, window + rq)
-        nsplit = max(1, min(want, 32, span // 64))
+        nsplit, warps, _ = stream_split(NB * Hkv, span, lib().mary_sm_count())
     out = _empty(T, Hq, D, dtype=torch.bfloat16, device=q.device)
-    scratch = None
-    if nsplit > 1:
-        scratch = _empty(lib().mary_paged_attention_scratch_floats(NB, Hkv, nsplit, D), dtype=torch.float32, device=q.device)
-    kc, vc = kcache.codes, vcache.codes
-    check(lib().mary_paged_attention_decode_q8(_p(q.contiguous()), _p(kc), _p(vc), _p(kcache.sz), _p(vcache.sz), _p(out), _p(meta.page_table),
-                                               _p(meta.kv_len), _p(meta.q_start), _p(blk_seq), _p(blk_q0), NB, meta.page_table.shape[1],
-                                               meta.page_size, kc.stride(1), kc.stride(0), vc.stride(1), vc.stride(0), Hq, Hkv, D, rq,
-                                               nsplit, window, scale, softcap, _p(scratch), _stream()), "paged_attention_decode_q8")
+    q = q.contiguous()
+    check(lib().mary_attention_stream(_p(q), _p(kc), _p(vc), _p(kcache.sz) if q8 else None, _p(vcache.sz) if q8 else None, _p(out), _p(meta.page_table),
+                                      _p(meta.kv_len), _p(meta.q_start), _p(blk_seq), _p(blk_q0), NB, meta.page_table.shape[1], meta.page_size,
+                                      kc.stride(1), kc.stride(0), vc.stride(1), vc.stride(0), q.stride(0), Hq * D, Hq, Hkv, D, rq, nsplit, warps or 4,
+                                      window, scale, softcap, _stream()), "attention_stream")
     return out
 
 
@@ -647,6 +696,9 @@ def paged_attention(q, kcache, vcache, meta, scale, window=0, softcap=0.0, dv: i
             and lib().mary_attention_prefill_supported(DK, DV) and q.dtype == torch.bfloat16 \
             and (kernel == "prefill" or T >= PREFILL_MIN_ROWS * meta.num_seqs):
         return attention_prefill(q, kcache, vcache, meta, scale, window)
+    if kernel == "auto" and GQA_TC and dv is None and q.dtype == torch.bfloat16 and kcache.dtype == torch.bfloat16 and kcache.dim() == 4 and DK == DV \
+            and _stream_wins(q, kcache, vcache, meta, window):
+        return attention_stream(q, kcache, vcache, meta, scale, window, softcap)
     if kernel in ("auto", "tc") and (kernel == "tc" or GQA_TC) and dv is None and gqa_tc_supported(q, kcache, meta):
         return gqa_decode_tc(q, kcache, vcache, meta, scale, window, softcap, nsplit)
     if kernel == "tc":
