@@ -74,19 +74,21 @@ __global__ void argmax_kernel(const float* __restrict__ logits, int64_t ld, int 
 // `n_group` groups (group score = sum of its two best biased scores); weights = unbiased scores of the chosen,
 // renormalised by (sum + 1e-20), times `scale`.  Ties resolve to the lower index.  A non-finite logit sets *flag.
 constexpr int MAXE_PER_LANE = 16;   // up to 512 experts
+template <int PER>                  // experts per lane at most
 __global__ void router_topk_kernel(const float* __restrict__ logits, int64_t ld, const float* __restrict__ bias, int T, int E, int k,
                                    int mode, int n_group, int topk_group, float scale, int renorm, int* __restrict__ out_idx,
                                    float* __restrict__ out_w, int* __restrict__ counts, int* __restrict__ flag) {
+  pdl_sync();
   const int t = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (t >= T) return;
   const int lane = threadIdx.x & 31;
   const float* row = logits + (int64_t)t * ld;
-  float sc[MAXE_PER_LANE], sel[MAXE_PER_LANE];
+  float sc[PER], sel[PER];
   const int per = (E + 31) / 32;
   float mx = -INFINITY;
   bool bad = false;
 #pragma unroll
-  for (int j = 0; j < MAXE_PER_LANE; ++j) {
+  for (int j = 0; j < PER; ++j) {
     const int e = lane + 32 * j;
     sc[j] = -INFINITY;
     if (j < per && e < E) { sc[j] = row[e]; bad |= !isfinite(sc[j]); mx = fmaxf(mx, sc[j]); }
@@ -96,19 +98,19 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, int64_t ld,
     mx = warp_max(mx);
     float sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < MAXE_PER_LANE; ++j) {
+    for (int j = 0; j < PER; ++j) {
       const int e = lane + 32 * j;
       if (j < per && e < E) { sc[j] = __expf(sc[j] - mx); sum += sc[j]; } else sc[j] = -INFINITY;
     }
     sum = warp_sum(sum);
 #pragma unroll
-    for (int j = 0; j < MAXE_PER_LANE; ++j) {
+    for (int j = 0; j < PER; ++j) {
       if (sc[j] != -INFINITY) sc[j] /= sum;
       sel[j] = sc[j] + (bias && lane + 32 * j < E ? bias[lane + 32 * j] : 0.f);
     }
   } else {
 #pragma unroll
-    for (int j = 0; j < MAXE_PER_LANE; ++j) {
+    for (int j = 0; j < PER; ++j) {
       const int e = lane + 32 * j;
       if (j < per && e < E) { sc[j] = 1.0f / (1.0f + __expf(-sc[j])); sel[j] = sc[j] + (bias ? bias[e] : 0.f); }
       else { sc[j] = 0.f; sel[j] = -INFINITY; }
@@ -121,11 +123,11 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, int64_t ld,
       for (int g = 0; g < n_group; ++g) {
         MaxIdx b1{-INFINITY, 0x7fffffff};
 #pragma unroll
-        for (int j = 0; j < MAXE_PER_LANE; ++j) { const int e = lane + 32 * j; if (j < per && e < E && e / gsz == g) b1 = better(b1, MaxIdx{sel[j], e}); }
+        for (int j = 0; j < PER; ++j) { const int e = lane + 32 * j; if (j < per && e < E && e / gsz == g) b1 = better(b1, MaxIdx{sel[j], e}); }
         b1 = warp_best(b1);
         MaxIdx b2{-INFINITY, 0x7fffffff};
 #pragma unroll
-        for (int j = 0; j < MAXE_PER_LANE; ++j) { const int e = lane + 32 * j; if (j < per && e < E && e / gsz == g && e != b1.i) b2 = better(b2, MaxIdx{sel[j], e}); }
+        for (int j = 0; j < PER; ++j) { const int e = lane + 32 * j; if (j < per && e < E && e / gsz == g && e != b1.i) b2 = better(b2, MaxIdx{sel[j], e}); }
         b2 = warp_best(b2);
         if (lane == g) gscore_mine = b1.v + b2.v;
       }
@@ -134,7 +136,7 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, int64_t ld,
         keep |= 1u << b.i;
       }
 #pragma unroll
-      for (int j = 0; j < MAXE_PER_LANE; ++j) { const int e = lane + 32 * j; if (j < per && e < E && !((keep >> (e / gsz)) & 1u)) sel[j] = -INFINITY; }
+      for (int j = 0; j < PER; ++j) { const int e = lane + 32 * j; if (j < per && e < E && !((keep >> (e / gsz)) & 1u)) sel[j] = -INFINITY; }
     }
   }
   float wsum = 0.f, mine_w = 0.f;
@@ -142,12 +144,12 @@ __global__ void router_topk_kernel(const float* __restrict__ logits, int64_t ld,
   for (int r = 0; r < k; ++r) {
     MaxIdx b{-INFINITY, 0x7fffffff};
 #pragma unroll
-    for (int j = 0; j < MAXE_PER_LANE; ++j) { const int e = lane + 32 * j; if (j < per && e < E) b = better(b, MaxIdx{sel[j], e}); }
+    for (int j = 0; j < PER; ++j) { const int e = lane + 32 * j; if (j < per && e < E) b = better(b, MaxIdx{sel[j], e}); }
     b = warp_best(b);
     // the owning lane reads the unbiased score and retires the expert
     float wv = 0.f;
 #pragma unroll
-    for (int j = 0; j < MAXE_PER_LANE; ++j) { if (lane + 32 * j == b.i) { wv = sc[j]; sel[j] = -INFINITY; } }
+    for (int j = 0; j < PER; ++j) { if (lane + 32 * j == b.i) { wv = sc[j]; sel[j] = -INFINITY; } }
     wv = __shfl_sync(0xffffffffu, wv, b.i & 31);
     wsum += wv;
     if (lane == r) { mine_w = wv; mine_i = b.i; }
@@ -193,16 +195,23 @@ MARY_API int mary_router_topk(const float* logits, int64_t ld, const float* bias
                               cudaStream_t s) {
   if (T <= 0) return MARY_OK;
   if (E > 32 * MAXE_PER_LANE || k > 32 || n_group > 32 || (n_group > 1 && E % n_group)) return MARY_ERR_BAD_ARG;
-  if (T <= 16384 && k * 8 <= 256) {
-    // one CTA per token: short dependent chains (decode and ordinary prefill chunks)
+  // One CTA per token has the shorter chain, one warp per token an eighth of the instructions: 256 tokens of 128 experts take 6.0 us by CTAs and 4.3 by
+  // warps, 4096 take 34 and 7.6.  Groups, or more experts than 8 per lane, make the warp's chain the longer one: 384 experts in 8 groups take 16 us by
+  // CTAs and 37 by warps at 1024 tokens.
+  const bool warps = n_group <= 1 && E <= 256 && T >= 256;
+  if (!warps && T <= 16384 && k * 8 <= 256) {
     MARY_LAUNCH(router_topk_block_kernel, T, 256, 0, s, logits, ld, bias, T, E, k, mode, n_group, topk_group, scale, renorm, out_idx, out_w,
                                                counts, flag);
     MARY_CHECK_LAUNCH();
     return MARY_OK;
   }
   const int wpb = 4;
-  router_topk_kernel<<<(T + wpb - 1) / wpb, wpb * 32, 0, s>>>(logits, ld, bias, T, E, k, mode, n_group, topk_group, scale, renorm,
-                                                            out_idx, out_w, counts, flag);
+#define MARY_ROUTE(PER_) MARY_LAUNCH((router_topk_kernel<PER_>), (T + wpb - 1) / wpb, wpb * 32, 0, s, logits, ld, bias, T, E, k, mode, n_group, topk_group, \
+                                     scale, renorm, out_idx, out_w, counts, flag)
+  if (E <= 32 * 4) MARY_ROUTE(4);
+  else if (E <= 32 * 8) MARY_ROUTE(8);
+  else MARY_ROUTE(16);
+#undef MARY_ROUTE
   MARY_CHECK_LAUNCH();
   return MARY_OK;
 }
