@@ -26,6 +26,7 @@
 
 #include "common.cuh"
 #include "host_utils.h"
+#include "nvfp4_quant.cuh"
 
 using namespace mary;
 
@@ -102,12 +103,6 @@ __global__ void ep_plan_kernel(const int* __restrict__ cm, int world, int rank, 
   }
 }
 
-__device__ __forceinline__ uint32_t e2m1_code(float y) {
-  const float m = fabsf(y);
-  uint32_t c = (m >= 0.25f) + (m >= 0.75f) + (m >= 1.25f) + (m >= 1.75f) + (m >= 2.5f) + (m >= 3.5f) + (m >= 5.0f);
-  return c | (signbit(y) ? 8u : 0u);
-}
-
 // One CTA per entry i = t * k + j.
 __global__ void ep_dispatch_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int* __restrict__ idx, int k, int E, int e_local,
                                    int Kd, int NT, int rank, int entry_stride, int cap_rows, const int* __restrict__ send_base,
@@ -132,27 +127,9 @@ __global__ void ep_dispatch_kernel(const __nv_bfloat16* __restrict__ x, int64_t 
   const int64_t sf_base = (int64_t)tile * (Kd / 64) * 512 + (r % 32) * 16 + (r / 32) * 4;
   for (int b = threadIdx.x; b < Kd / 16; b += blockDim.x) {
     const uint4 v0 = *(const uint4*)(xr + b * 16), v1 = *(const uint4*)(xr + b * 16 + 8);
-    float f[16];
-    const __nv_bfloat162* p0 = (const __nv_bfloat162*)&v0;
-    const __nv_bfloat162* p1 = (const __nv_bfloat162*)&v1;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float2 a = __bfloat1622float2(p0[j]), c = __bfloat1622float2(p1[j]);
-      f[2 * j] = a.x; f[2 * j + 1] = a.y; f[8 + 2 * j] = c.x; f[8 + 2 * j + 1] = c.y;
-    }
-    float amax = 0.f;
-#pragma unroll
-    for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
-    const float sfv = fminf(__fdiv_rn(amax, 6.0f), 448.0f);
-    const __nv_fp8_storage_t sb = __nv_cvt_float_to_fp8(sfv, __NV_SATFINITE, __NV_E4M3);
-    const float s = __half2float(__half(__nv_cvt_fp8_to_halfraw(sb, __NV_E4M3)));
-    uint32_t lo = 0, hi = 0;
-    if (s > 0.f) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) { lo |= e2m1_code(__fdiv_rn(f[j], s)) << (4 * j); hi |= e2m1_code(__fdiv_rn(f[8 + j], s)) << (4 * j); }
-    }
-    *(uint2*)(xq + (int64_t)row * (Kd / 2) + b * 8) = make_uint2(lo, hi);
-    sf[sf_base + (int64_t)(b / 4) * 512 + (b % 4)] = (uint8_t)sb;
+    uint8_t sb;
+    *(uint2*)(xq + (int64_t)row * (Kd / 2) + b * 8) = nvfp4_block16(v0, v1, &sb);
+    sf[sf_base + (int64_t)(b / 4) * 512 + (b % 4)] = sb;
   }
 }
 

@@ -52,27 +52,9 @@ ep_route_dispatch_kernel(const RouteParams p, const EpCtx c) {
     const __nv_bfloat16* xr = p.x + (int64_t)t * p.ldx;
     for (int b = tid; b < p.H / 16; b += blockDim.x) {
       const uint4 v0 = *(const uint4*)(xr + b * 16), v1 = *(const uint4*)(xr + b * 16 + 8);
-      float f[16];
-      const __nv_bfloat162* p0 = (const __nv_bfloat162*)&v0;
-      const __nv_bfloat162* p1 = (const __nv_bfloat162*)&v1;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        float2 a = __bfloat1622float2(p0[j]), q = __bfloat1622float2(p1[j]);
-        f[2 * j] = a.x; f[2 * j + 1] = a.y; f[8 + 2 * j] = q.x; f[8 + 2 * j + 1] = q.y;
-      }
-      float amax = 0.f;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
-      const float sfv = fminf(__fdiv_rn(amax, 6.0f), 448.0f);
-      const __nv_fp8_storage_t sb = __nv_cvt_float_to_fp8(sfv, __NV_SATFINITE, __NV_E4M3);
-      const float s = __half2float(__half(__nv_cvt_fp8_to_halfraw(sb, __NV_E4M3)));
-      uint32_t lo = 0, hi = 0;
-      if (s > 0.f) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) { lo |= nvfp4_code(__fdiv_rn(f[j], s)) << (4 * j); hi |= nvfp4_code(__fdiv_rn(f[8 + j], s)) << (4 * j); }
-      }
-      s_codes[b] = make_uint2(lo, hi);
-      s_sf[b] = (uint8_t)sb;
+      uint8_t sb;
+      s_codes[b] = nvfp4_block16(v0, v1, &sb);
+      s_sf[b] = sb;
     }
     router_block(p.logits + (int64_t)t * p.ld, p.bias, p.E, p.k, p.mode, p.n_group, p.topk_group, p.scale, p.renorm, S, p.flag);
     if (tid < K1) {

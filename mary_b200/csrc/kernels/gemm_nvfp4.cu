@@ -20,7 +20,11 @@
 //   * with GLU the CTA loads the gate tile and the matching up tile (rows n0 and F + n0), keeps two accumulators and
 //     writes act(gate) * up, so the [rows, 2F] intermediate never exists;
 //   * persistent CTAs, TMA producer warp / MMA warp / 4 epilogue warps, ring of stages, bounded waits;
-//   * the GLU epilogue can write its result ALREADY QUANTISED for the next GEMM (codes + scale tile): a thread holds one
+//   * 128-token tiles are turned in shared memory: a thread of the accumulator holds one feature of every token, so plain stores would be 2 bytes wide and
+//     a scale block would sit in 16 threads.  From the turned tile a thread quantises whole blocks and half a warp stores a row; with GLU, whose two
+//     accumulators fill TMEM, the main loop of the next tile starts before that.  4096 tokens of 8 among 128 experts, hidden 4096, width 1536: w13
+//     590 us + 71 us for the quantiser -> 283 us with it inside, w2 266 -> 195 us;
+//   * with 32-token tiles the GLU epilogue can write its result ALREADY QUANTISED for the next GEMM (codes + scale tile): a thread holds one
 //     feature of 32 token rows, so the 16-feature amax is a half-warp shuffle reduction and 8 codes pack into a word with
 //     three more shuffles — the separate quantiser pass between w13 and w2 disappears;
 //   * counter mode (ep_ctx.cuh): instead of a tile list from a planning kernel, every CTA waits (bounded) for the source
@@ -78,10 +82,22 @@ struct Cfg {
   static constexpr int ACC_BUFS = (2 * ACC_COLS + SF_COLS <= 512) ? 2 : 1;
   static constexpr int COLS_RAW = ACC_BUFS * ACC_COLS + SF_COLS;
   static constexpr int TMEM_COLS = COLS_RAW <= 32 ? 32 : COLS_RAW <= 64 ? 64 : COLS_RAW <= 128 ? 128 : COLS_RAW <= 256 ? 256 : 512;
-  static constexpr int STAGES_RAW = (219 * 1024) / STAGE_BYTES;
+  // 128-token tiles leave through a bf16 tile [token][feature] in shared memory, its rows 16 bytes apart in the banks
+  static constexpr bool TURN = NT == 128;
+  static constexpr int TURN_PITCH = BM * 2 + 16;
+  static constexpr int TURN_BYTES = TURN ? NT * TURN_PITCH : 0;
+  static constexpr int STAGES_RAW = (219 * 1024 - TURN_BYTES) / STAGE_BYTES;
   static constexpr int STAGES = STAGES_RAW > 10 ? 10 : STAGES_RAW;
-  static constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+  static constexpr int SMEM = STAGES * STAGE_BYTES + TURN_BYTES + 1024 + 256;
 };
+
+// The 128 epilogue threads meet; true when `ok` holds in all of them.
+__device__ __forceinline__ bool epilogue_meet(bool ok) {
+  int all;
+  asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, 1, 128, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+               : "=r"(all) : "r"((int)ok) : "memory");
+  return all != 0;
+}
 
 template <int NT, bool GLU>
 __global__ void __launch_bounds__(NTHREADS, 1)
@@ -94,7 +110,8 @@ gemm_nvfp4_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
   __shared__ int s_ntiles;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~uintptr_t(1023));
-  uint64_t* full = (uint64_t*)(smem + C::STAGES * C::STAGE_BYTES);
+  uint8_t* const turned = smem + C::STAGES * C::STAGE_BYTES;
+  uint64_t* full = (uint64_t*)(turned + C::TURN_BYTES);
   uint64_t* empty = full + C::STAGES;
   uint64_t* acc_full = empty + C::STAGES;
   uint64_t* acc_empty = acc_full + 2;
@@ -240,11 +257,77 @@ gemm_nvfp4_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
       const int wt = WT_FAST ? w % p.w_tiles : w / n_tiles;
       const int buf = C::ACC_BUFS == 2 ? (it & 1) : 0;
       const uint32_t acc_phase = C::ACC_BUFS == 2 ? ((it >> 1) & 1) : (it & 1);
-      if (!mbar_wait(&acc_full[buf], acc_phase, abort_flag, p.status, MARY_ERR_TIMEOUT_MMA)) goto done;
+      const bool ok = mbar_wait(&acc_full[buf], acc_phase, abort_flag, p.status, MARY_ERR_TIMEOUT_MMA);
+      // 128-token tiles: the four warps go on, or leave, together, and none refills the turned tile before all have emptied it
+      if constexpr (C::TURN) { if (!epilogue_meet(ok)) goto done; }
+      else if (!ok) goto done;
       tc_fence_after();
       const float s2 = p.scale2[t.expert];
       const int n = wt * BM + q * 32 + lane;                // output feature of this thread
       const uint32_t taddr = tmem_base + buf * C::ACC_COLS + ((uint32_t)(q * 32) << 16);
+      if constexpr (C::TURN) {
+        // this thread's feature of every token -> bf16 -> the turned tile; the accumulator is free for the next tile's main loop before the rows are
+        // quantised or stored
+        __nv_bfloat16* const col = (__nv_bfloat16*)(turned + (q * 32 + lane) * 2);
+#pragma unroll 1
+        for (int c0 = 0; c0 < t.rows; c0 += 32) {
+          uint32_t r[32], r2[32];
+          tmem_ld_32x32b_x32(taddr + c0, r);
+          if (GLU) tmem_ld_32x32b_x32(taddr + NT + c0, r2);
+          tmem_ld_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) {
+            const float a = __uint_as_float(r[j]) * s2;
+            col[(c0 + j) * (C::TURN_PITCH / 2)] = __float2bfloat16(GLU ? glu_f(p.act, a, __uint_as_float(r2[j]) * s2) : a);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&acc_empty[buf]);
+        epilogue_meet(true);
+        if (GLU && p.q_out) {
+          // thread = token: the 128 features as codes and scale bytes for the next GEMM
+          const int rr = threadIdx.x - 64;
+          if (rr < t.rows) {
+            const uint4* src = (const uint4*)(turned + rr * C::TURN_PITCH);
+            uint8_t* codes = p.q_out + (int64_t)(t.row0 + rr) * (p.n_out / 2) + wt * (BM / 2);
+            uint8_t* scales = p.q_sf + ((int64_t)t.sf_tile * (p.n_out / 64) + wt * 2) * 512 + (rr % 32) * 16 + (rr / 32) * 4;
+#pragma unroll
+            for (int g = 0; g < 2; ++g) {
+              uint2 c[4];
+              uint32_t four = 0;
+#pragma unroll
+              for (int b = 0; b < 4; ++b) {
+                uint8_t sb;
+                c[b] = nvfp4_block16(src[g * 8 + 2 * b], src[g * 8 + 2 * b + 1], &sb);
+                four |= (uint32_t)sb << (8 * b);
+              }
+              *(uint4*)(codes + g * 32) = make_uint4(c[0].x, c[0].y, c[1].x, c[1].y);
+              *(uint4*)(codes + g * 32 + 16) = make_uint4(c[2].x, c[2].y, c[3].x, c[3].y);
+              *(uint32_t*)(scales + g * 512) = four;
+            }
+          }
+        } else {
+          // half a warp per token row: 256 bytes
+          const int part = lane & 15;
+#pragma unroll 4
+          for (int i = 0; i < 16; ++i) {
+            const int rr = q * 32 + 2 * i + (lane >> 4);
+            if (rr >= t.rows) break;
+            __nv_bfloat16* dst = p.row_ptrs ? (__nv_bfloat16*)p.row_ptrs[t.row0 + rr] : p.out + (int64_t)(t.row0 + rr) * p.ldo;
+            if (!dst) continue;
+            dst += wt * BM + part * 8;
+            const uint4 v = *(const uint4*)(turned + rr * C::TURN_PITCH + part * 16);
+            if (((uintptr_t)dst & 15) == 0) *(uint4*)dst = v;
+            else {
+              const __nv_bfloat16* e = (const __nv_bfloat16*)&v;
+#pragma unroll
+              for (int j = 0; j < 8; ++j) dst[j] = e[j];
+            }
+          }
+        }
+        continue;
+      }
 #pragma unroll 1
       for (int c0 = 0; c0 < NT; c0 += 32) {
         if (c0 >= t.rows) break;
@@ -260,6 +343,7 @@ gemm_nvfp4_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
             const int64_t sf_base = (int64_t)t.sf_tile * (p.n_out / 64) * 512 + (int64_t)(n / 64) * 512 + ((n / 16) & 3);
 #pragma unroll
             for (int j = 0; j < 32; ++j) {
+              if (c0 + j >= t.rows) break;                     // the same in every lane
               const float a = __uint_as_float(r[j]) * s2;
               const float v = __bfloat162float(__float2bfloat16(glu_f(p.act, a, __uint_as_float(r2[j]) * s2)));
               float amax = fabsf(v);
@@ -269,15 +353,13 @@ gemm_nvfp4_grouped_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid
               amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 8));
               float s;
               const uint8_t sb = nvfp4_scale_byte(amax, &s);
-              uint32_t pk = (s > 0.f ? nvfp4_code(__fdiv_rn(v, s)) : 0u) << (4 * sub);
+              uint32_t pk = (s > 0.f ? nvfp4_pair(nvfp4_quotient(v, nvfp4_inverse(s)), 0.f) : 0u) << (4 * sub);
               pk |= __shfl_xor_sync(0xffffffffu, pk, 1);
               pk |= __shfl_xor_sync(0xffffffffu, pk, 2);
               pk |= __shfl_xor_sync(0xffffffffu, pk, 4);
-              if (c0 + j < t.rows) {
-                const int rr = c0 + j;                         // row within the tile
-                if (sub == 0) *(uint32_t*)(p.q_out + (int64_t)(t.row0 + rr) * (p.n_out / 2) + n / 2) = pk;
-                if ((lane & 15) == 0) p.q_sf[sf_base + (rr % 32) * 16 + (rr / 32) * 4] = sb;
-              }
+              const int rr = c0 + j;                           // row within the tile
+              if (sub == 0) *(uint32_t*)(p.q_out + (int64_t)(t.row0 + rr) * (p.n_out / 2) + n / 2) = pk;
+              if ((lane & 15) == 0) p.q_sf[sf_base + (rr % 32) * 16 + (rr / 32) * 4] = sb;
             }
           } else {
             // destination of every row: plain output, a caller-given address list, or (counter mode 2) the combine slot of the

@@ -12,6 +12,7 @@
 
 #include "common.cuh"
 #include "host_utils.h"
+#include "nvfp4_quant.cuh"
 
 using namespace mary;
 
@@ -19,29 +20,66 @@ namespace {
 
 struct Tile { int expert, row0, rows, sf_tile; };
 
-// One CTA.  idx[n_entries] = expert of every (token, slot) entry (negative = entry not routed here).
+__device__ __forceinline__ void cluster_meet() { asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ int ld_cluster_int(const int* p, uint32_t rank) {
+  uint32_t a;
+  int v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+
+// One cluster of 1 to 8 CTAs.  idx[n_entries] = expert of every (token, slot) entry (negative = entry not routed here).
 // Outputs: row_of[n_entries] padded row of each entry (-1 if skipped), src_of[max_rows] token of each padded row
 // (-1 for padding), tiles/n_tiles for the grouped GEMM, counts[E], meta = {n_tiles, padded rows}.
-__global__ void moe_plan_kernel(const int* __restrict__ idx, int n_entries, int k, int E, int NT, int max_rows, int* __restrict__ row_of,
-                                int* __restrict__ src_of, Tile* __restrict__ tiles, int* __restrict__ meta, int* __restrict__ counts_out) {
+// Bound: the shared-memory counters (an atomic per entry, whose old value is the slot) and one load latency per chunk.  Each CTA of the cluster counts its
+// run of entries, and learns from the others' counters where its slots start in each expert: 48 us for 32768 entries in one CTA that met at a barrier
+// after every 1024.
+constexpr int PLAN_CHUNK = 4;                  // entries a thread loads before it counts the first
+__global__ void __launch_bounds__(1024)
+moe_plan_kernel(const int* __restrict__ idx, int n_entries, int k, int E, int NT, int max_rows, int* __restrict__ row_of,
+                int* __restrict__ src_of, Tile* __restrict__ tiles, int* __restrict__ meta, int* __restrict__ counts_out) {
   pdl_sync();
   extern __shared__ int sh[];
-  int* cnt = sh;            // [E]
-  int* off = sh + E;        // [E + 1]
+  int* cnt = sh;            // [E] of this CTA
+  int* off = sh + E;        // [E + 1] first padded row of an expert
+  int* start = off + E + 1; // [E] this CTA's first slot in an expert
+  int* all = start + E;     // [E] entries of an expert
+  const int ctas = gridDim.x, rank = blockIdx.x;
+  const int run = ((n_entries + ctas - 1) / ctas + 3) / 4 * 4, lo = min(n_entries, rank * run), hi = min(n_entries, lo + run);
   for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0;
-  for (int r = threadIdx.x; r < max_rows; r += blockDim.x) src_of[r] = -1;
+  for (int r = rank * blockDim.x + threadIdx.x; r < max_rows; r += ctas * blockDim.x) src_of[r] = -1;
   __syncthreads();
-  // Slots inside an expert come from a shared-memory counter.  Their order within a chunk of blockDim entries
-  // depends on scheduling, which does not matter: every row of the grouped GEMM is independent and the un-permute
-  // sums a token's k results in fixed slot order.
-  for (int base = 0; base < n_entries; base += blockDim.x) {
-    const int i = base + threadIdx.x;
-    const int e = (i < n_entries) ? idx[i] : -1;
-    int slot = -1;
-    if (e >= 0 && e < E) slot = atomicAdd(&cnt[e], 1);      // (a warp-aggregated form with match.any measured slower: 108 against 70 us)
-    if (i < n_entries) row_of[i] = slot;       // provisional: slot inside the expert
-    __syncthreads();
+  // Slots inside an expert come from a shared-memory counter.  Their order inside a CTA's run depends on scheduling, which does not matter: every row of
+  // the grouped GEMM is independent and the un-permute sums a token's k results in fixed slot order.
+  // (A warp-aggregated form with match.any measured slower: 108 against 70 us.)
+  for (int base = lo; base < hi; base += blockDim.x * PLAN_CHUNK) {
+    int e[PLAN_CHUNK];
+#pragma unroll
+    for (int j = 0; j < PLAN_CHUNK; ++j) {
+      const int i = base + j * blockDim.x + threadIdx.x;
+      e[j] = i < hi ? idx[i] : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < PLAN_CHUNK; ++j) {
+      const int i = base + j * blockDim.x + threadIdx.x;
+      const int slot = e[j] >= 0 && e[j] < E ? atomicAdd(&cnt[e[j]], 1) : -1;
+      if (i < hi) row_of[i] = slot;            // provisional: slot inside the expert and this CTA's run
+    }
   }
+  __syncthreads();
+  if (ctas > 1) cluster_meet();                // every CTA's counters are final
+  for (int e = threadIdx.x; e < E; e += blockDim.x) {
+    int before = 0, sum = 0;
+    for (int r = 0; r < ctas; ++r) {
+      const int c = ctas > 1 ? ld_cluster_int(cnt + e, r) : cnt[e];
+      before += r < rank ? c : 0;
+      sum += c;
+    }
+    start[e] = before;
+    all[e] = sum;
+  }
+  __syncthreads();
   // exclusive prefix sum of the padded counts as a block scan (warp shuffles + one pass over the warp totals)
   {
     __shared__ int warp_tot[33];
@@ -51,7 +89,7 @@ __global__ void moe_plan_kernel(const int* __restrict__ idx, int n_entries, int 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     for (int base = 0; base < E; base += blockDim.x) {
       const int e = base + threadIdx.x;
-      const int padded = e < E ? (cnt[e] + NT - 1) / NT * NT : 0;
+      const int padded = e < E ? (all[e] + NT - 1) / NT * NT : 0;
       int incl = padded;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) { const int v = __shfl_up_sync(0xffffffffu, incl, o); if (lane >= o) incl += v; }
@@ -72,31 +110,37 @@ __global__ void moe_plan_kernel(const int* __restrict__ idx, int n_entries, int 
       if (threadIdx.x == 0) carry_s += warp_tot[32];
       __syncthreads();
     }
-    if (threadIdx.x == 0) { off[E] = carry_s; meta[0] = carry_s / NT; meta[1] = carry_s; }
+    if (threadIdx.x == 0) { off[E] = carry_s; if (rank == 0) { meta[0] = carry_s / NT; meta[1] = carry_s; } }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    if (counts_out) counts_out[e] = cnt[e];
-    const int c = cnt[e];
+  for (int e = rank * blockDim.x + threadIdx.x; e < E; e += ctas * blockDim.x) {
+    if (counts_out) counts_out[e] = all[e];
+    const int c = all[e];
     for (int i = 0; i * NT < c; ++i) {
       Tile t{e, off[e] + i * NT, min(NT, c - i * NT), off[e] / NT + i};
       tiles[off[e] / NT + i] = t;
     }
   }
-  for (int i = threadIdx.x; i < n_entries; i += blockDim.x) {
-    const int e = idx[i];
-    if (e >= 0 && e < E) {
-      const int row = off[e] + row_of[i];
-      row_of[i] = row;
-      src_of[row] = i / k;
-    } else row_of[i] = -1;
+  for (int base = lo; base < hi; base += blockDim.x * PLAN_CHUNK) {
+    int e[PLAN_CHUNK], slot[PLAN_CHUNK];
+#pragma unroll
+    for (int j = 0; j < PLAN_CHUNK; ++j) {
+      const int i = base + j * blockDim.x + threadIdx.x;
+      e[j] = i < hi ? idx[i] : -1;
+      slot[j] = i < hi ? row_of[i] : -1;
+    }
+#pragma unroll
+    for (int j = 0; j < PLAN_CHUNK; ++j) {
+      const int i = base + j * blockDim.x + threadIdx.x;
+      if (i >= hi) continue;
+      if (e[j] >= 0 && e[j] < E) {
+        const int row = off[e[j]] + start[e[j]] + slot[j];
+        row_of[i] = row;
+        src_of[row] = i / k;
+      } else row_of[i] = -1;
+    }
   }
-}
-
-__device__ __forceinline__ uint32_t e2m1_code(float y) {
-  const float m = fabsf(y);
-  uint32_t c = (m >= 0.25f) + (m >= 0.75f) + (m >= 1.25f) + (m >= 1.75f) + (m >= 2.5f) + (m >= 3.5f) + (m >= 5.0f);
-  return c | (signbit(y) ? 8u : 0u);
+  if (ctas > 1) cluster_meet();                // the counters stay until every CTA has read them
 }
 
 // One CTA per destination row.  src_of[row] < 0 -> padding row, skipped.  identity != 0 -> the source row is `row`
@@ -104,32 +148,6 @@ __device__ __forceinline__ uint32_t e2m1_code(float y) {
 // Scales go to the 512-byte block layout of the row's NT-row tile; optionally also row-major (tests, dense users).
 // With row_of (entry -> padded row, k entries per token) the grid runs over the ENTRIES instead of the padded rows: a decode
 // batch has a few hundred entries but thousands of padded rows, most of them padding.
-// 16 consecutive values -> 8 code bytes and the scale byte of their block
-__device__ __forceinline__ uint2 nvfp4_block16(const __nv_bfloat16* __restrict__ src, uint8_t* sb_out) {
-  const uint4 v0 = *(const uint4*)src, v1 = *(const uint4*)(src + 8);
-  float f[16];
-  const __nv_bfloat162* p0 = (const __nv_bfloat162*)&v0;
-  const __nv_bfloat162* p1 = (const __nv_bfloat162*)&v1;
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    float2 a = __bfloat1622float2(p0[j]), c = __bfloat1622float2(p1[j]);
-    f[2 * j] = a.x; f[2 * j + 1] = a.y; f[8 + 2 * j] = c.x; f[8 + 2 * j + 1] = c.y;
-  }
-  float amax = 0.f;
-#pragma unroll
-  for (int j = 0; j < 16; ++j) amax = fmaxf(amax, fabsf(f[j]));
-  const float sfv = fminf(__fdiv_rn(amax, 6.0f), 448.0f);
-  const __nv_fp8_storage_t sb = __nv_cvt_float_to_fp8(sfv, __NV_SATFINITE, __NV_E4M3);
-  const float s = __half2float(__half(__nv_cvt_fp8_to_halfraw(sb, __NV_E4M3)));
-  uint32_t lo = 0, hi = 0;
-  if (s > 0.f) {
-#pragma unroll
-    for (int j = 0; j < 8; ++j) { lo |= e2m1_code(__fdiv_rn(f[j], s)) << (4 * j); hi |= e2m1_code(__fdiv_rn(f[8 + j], s)) << (4 * j); }
-  }
-  *sb_out = (uint8_t)sb;
-  return make_uint2(lo, hi);
-}
-
 __global__ void quant_nvfp4_rows_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx, const int* __restrict__ src_of, int identity,
                                         int Kd, int NT, uint8_t* __restrict__ xq, uint8_t* __restrict__ sf_tiles,
                                         uint8_t* __restrict__ sf_rowmajor, const int* __restrict__ n_rows,
@@ -150,7 +168,7 @@ __global__ void quant_nvfp4_rows_kernel(const __nv_bfloat16* __restrict__ x, int
   const int64_t sf_base = (int64_t)tile * (Kd / 64) * 512 + (r % 32) * 16 + (r / 32) * 4;
   for (int b = threadIdx.x; b < Kd / 16; b += blockDim.x) {
     uint8_t sb;
-    const uint2 code = nvfp4_block16(xr + b * 16, &sb);
+    const uint2 code = nvfp4_block16(*(const uint4*)(xr + b * 16), *(const uint4*)(xr + b * 16 + 8), &sb);
     *(uint2*)(xq + (int64_t)row * (Kd / 2) + b * 8) = code;
     if (sf_tiles) sf_tiles[sf_base + (int64_t)(b / 4) * 512 + (b % 4)] = sb;
     if (sf_rowmajor) sf_rowmajor[(int64_t)row * (Kd / 16) + b] = sb;
@@ -174,14 +192,22 @@ __global__ void quant_nvfp4_tokens_kernel(const __nv_bfloat16* __restrict__ x, i
     sfb[j] = (int64_t)tile * (Kd / 64) * 512 + (r % 32) * 16 + (r / 32) * 4;
   }
   const __nv_bfloat16* xr = x + (int64_t)t * ldx;
-  for (int b = threadIdx.x; b < Kd / 16; b += blockDim.x) {
-    uint8_t sb;
-    const uint2 code = nvfp4_block16(xr + b * 16, &sb);
+  // four neighbouring lanes hold the blocks of 64 values, whose scale bytes are neighbours in the tile: one 4-byte store for the four
+  for (int b0 = 0; b0 < Kd / 16; b0 += blockDim.x) {          // Kd % 64 == 0: groups of four are whole
+    const int b = b0 + threadIdx.x;
+    const bool in = b < Kd / 16;
+    uint8_t sb = 0;
+    uint2 code = make_uint2(0, 0);
+    if (in) code = nvfp4_block16(*(const uint4*)(xr + b * 16), *(const uint4*)(xr + b * 16 + 8), &sb);
+    uint32_t four = (uint32_t)sb << (8 * (b & 3));
+    four |= __shfl_xor_sync(0xffffffffu, four, 1);
+    four |= __shfl_xor_sync(0xffffffffu, four, 2);
+    if (!in) continue;
 #pragma unroll
     for (int j = 0; j < K_ENT; ++j)
       if (rows[j] >= 0) {
         *(uint2*)(xq + (int64_t)rows[j] * (Kd / 2) + b * 8) = code;
-        sf_tiles[sfb[j] + (int64_t)(b / 4) * 512 + (b % 4)] = sb;
+        if ((b & 3) == 0) *(uint32_t*)(sf_tiles + sfb[j] + (int64_t)(b / 4) * 512) = four;
       }
   }
 }
@@ -225,7 +251,25 @@ __global__ void moe_unpermute_kernel(const __nv_bfloat16* __restrict__ y, int64_
 MARY_API int mary_moe_plan(const int* idx, int n_entries, int k, int E, int NT, int max_rows, int* row_of, int* src_of, void* tiles,
                            int* meta, int* counts, cudaStream_t s) {
   if (E > 4096 || NT <= 0) return MARY_ERR_BAD_ARG;
-  MARY_LAUNCH(moe_plan_kernel, 1, 1024, (2 * E + 1) * sizeof(int), s, idx, n_entries, k, E, NT, max_rows, row_of, src_of, (Tile*)tiles, meta, counts);
+  // one CTA up to 4096 entries (four per thread), then as many as keep each at that, at most a portable cluster
+  int ctas = 1;
+  while (ctas < 8 && n_entries > 4096 * ctas) ctas *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(1024);
+  cfg.dynamicSmemBytes = (4 * E + 1) * sizeof(int);
+  static MarySmemSlots smem_set = {};
+  if (int rc = mary_ensure_dyn_smem((const void*)moe_plan_kernel, cfg.dynamicSmemBytes, &smem_set)) return rc;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = mary_pdl_enabled() ? 2 : 1;
+  if (cudaLaunchKernelEx(&cfg, moe_plan_kernel, idx, n_entries, k, E, NT, max_rows, row_of, src_of, (Tile*)tiles, meta, counts) != cudaSuccess) return MARY_ERR_CUDA;
   MARY_CHECK_LAUNCH();
   return MARY_OK;
 }

@@ -79,9 +79,7 @@ def grouped_gemm(wq, sfw, scale2, xq, sfx, plan: Plan, n_out: int, K: int, E: in
 
 
 declare("mary_gemm_nvfp4_grouped_glu_q", "ppppppppp" + "iiiliis")
-# with 32-token tiles the w13 GEMM of ``experts_forward`` leaves its GLU result quantised (same bytes as GEMM -> bf16 ->
-# quantiser, one launch less).  With 128-token tiles the GEMM has one accumulator buffer and the longer epilogue stalls its main
-# loop (measured on a 4096-token prefill: +65 ms in the GEMMs against 10 ms saved), so the quantiser stays a launch of its own.
+# the w13 GEMM of ``experts_forward`` leaves its GLU result quantised (same bytes as GEMM -> bf16 -> quantiser, one launch less)
 def _glu_quant_default() -> bool:
     from ..utils import flags
     return bool(flags.get("MARY_MOE_GLU_QUANT"))
@@ -115,7 +113,7 @@ def experts_forward(x, idx, w, ex, shared=None, nt: int | None = None):
         nt = 32 if T * k <= 32 * ex.E else 128
     plan = moe_plan(idx, ex.E, nt)
     xq, sfx = quantize_entries(x, plan, k, identity=False)
-    if FUSED_GLU_QUANT and nt == 32:
+    if FUSED_GLU_QUANT:
         hq, sfh = grouped_gemm_glu_q(ex.w13_q, ex.w13_sf, ex.w13_s2, xq, sfx, plan, ex.F, ex.H, ex.E, ex.act)
     else:
         h = grouped_gemm(ex.w13_q, ex.w13_sf, ex.w13_s2, xq, sfx, plan, ex.F, ex.H, ex.E, ex.act)
