@@ -131,8 +131,14 @@ __global__ void act_rows_kernel(T* __restrict__ y, int64_t ld, int n, int64_t to
 
 __global__ void soft_cap_kernel(float* __restrict__ x, int64_t n, float cap) {
   pdl_sync();
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) x[i] = cap * tanhf(x[i] / cap);
+  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+  if (i + 4 <= n && ((uintptr_t)x & 15) == 0) {
+    float4 v = *(const float4*)(x + i);
+    v.x = cap * tanhf(v.x / cap); v.y = cap * tanhf(v.y / cap); v.z = cap * tanhf(v.z / cap); v.w = cap * tanhf(v.w / cap);
+    *(float4*)(x + i) = v;
+  } else {
+    for (int64_t j = i; j < n && j < i + 4; ++j) x[j] = cap * tanhf(x[j] / cap);
+  }
 }
 
 // One warp per (token, head) of a projection row: RMS norm of query and key heads (gains optional), queries to qo, keys and values
@@ -341,7 +347,7 @@ MARY_API int mary_act_rows(void* y, int64_t ld, int T_, int n, int act, int f32,
 MARY_API int mary_soft_cap(float* x, int64_t n, float cap, cudaStream_t s) {
   if (n <= 0) return MARY_OK;
   if (!(cap > 0.f)) return MARY_ERR_BAD_ARG;
-  MARY_LAUNCH(soft_cap_kernel, (unsigned)((n + NT - 1) / NT), NT, 0, s, x, n, cap);
+  MARY_LAUNCH(soft_cap_kernel, (unsigned)((n + 4 * NT - 1) / (4 * NT)), NT, 0, s, x, n, cap);
   MARY_CHECK_LAUNCH();
   return MARY_OK;
 }

@@ -189,6 +189,9 @@ class Gemma4Model(nn.Module):
         return self.embed if self.lm_head is None else self.lm_head
 
     def logits(self, x):
+        cap = self.cfg.final_logit_softcapping
+        if x.is_cuda and x.dim() == 2 and cap and cap > 0:          # the sums stay f32 and are capped in place
+            return ops.soft_cap(ops.linear_f32(x, self.head_weight()), cap)
         return ref.softcap(ops.linear(x, self.head_weight()).float(), self.cfg.final_logit_softcapping)
 
     def forward(self, ids, meta, cache, rows=None, soft=None):
