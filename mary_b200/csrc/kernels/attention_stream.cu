@@ -368,7 +368,9 @@ int launch(const StreamParams& p, int NB, cudaStream_t s) {
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
-  cfg.numAttrs = mary_pdl_enabled() ? 2 : 1;
+  // More CTAs than SMs start after their predecessor: placed while it drains they would crowd three deep onto the SMs that are free first (256 CTAs of
+  // 2048 bf16 keys: 80 us instead of 66).
+  cfg.numAttrs = mary_pdl_enabled() && (int64_t)p.nsplit * NB * p.Hkv <= mary_num_sms() ? 2 : 1;
   if (cudaLaunchKernelEx(&cfg, attn_stream_kernel<D, R, Q8, WARPS>, p) != cudaSuccess) return MARY_ERR_CUDA;
   MARY_CHECK_LAUNCH();
   return MARY_OK;
@@ -380,13 +382,16 @@ int launch_warps(const StreamParams& p, int NB, int warps, cudaStream_t s) {
 }
 template <int D, int R>
 int launch_cache(const StreamParams& p, int NB, int warps, cudaStream_t s) {
-  return p.k_sz ? launch_warps<D, R, true>(p, NB, warps, s) : launch_warps<D, R, false>(p, NB, warps, s);
+  if (p.k_sz) return launch_warps<D, R, true>(p, NB, warps, s);
+  if constexpr (D == 256 && R <= 2) return launch_warps<D, R, false>(p, NB, warps, s);       // the other bf16 shapes are the tensor-core kernel's
+  return MARY_ERR_BAD_ARG;
 }
 
 }  // namespace
 
 // q [T, Hq, D] bf16 with row pitch q_ld, caches [pages, page, Hkv, D] with token and page strides in elements (k_sz / v_sz null: bf16; else unsigned
-// codes with (scale, zero) per (slot, kv head)), out rows of out_ld elements.  D 64, 128 or 256; RQ * (Hq / Hkv) <= 4 (D 256) or 8; nsplit 1, 2, 4 or 8;
+// codes with (scale, zero) per (slot, kv head)), out rows of out_ld elements.  D 64, 128 or 256, RQ * (Hq / Hkv) <= 4 (D 256) or 8 for codes; D 256 and
+// RQ * (Hq / Hkv) <= 2 for bf16; nsplit 1, 2, 4 or 8;
 // warps 4 or 8.  Query blocks as in mary_paged_attention.
 MARY_API int mary_attention_stream(const void* q, const void* kc, const void* vc, const float* k_sz, const float* v_sz, void* out, const int* page_table,
                                    const int* kv_len, const int* q_start, const int* blk_seq, const int* blk_q0, int NB, int max_pages, int page_size,

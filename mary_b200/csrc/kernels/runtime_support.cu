@@ -99,7 +99,10 @@ int mary_ensure_dyn_smem(const void* func, size_t bytes, MarySmemSlots* slots) {
 
 static int g_pdl = -1;          // -1: not decided yet (the environment decides at the first launch)
 
+static thread_local int t_pdl = -1;   // -1: as the process is set; else the choice of the calling thread's present scope
+
 int mary_pdl_enabled() {
+  if (t_pdl >= 0) return t_pdl;
   if (g_pdl < 0) {
     const char* e = getenv("MARY_PDL");
     g_pdl = (e && e[0] == '1') ? 1 : 0;
@@ -111,3 +114,9 @@ int mary_pdl_enabled() {
 // gains from it, one with the expert pipeline in the chain loses: the caller that knows the model decides).  Graphs captured
 // before the call keep what they were captured with.
 MARY_API void mary_set_pdl(int on) { g_pdl = on ? 1 : 0; }
+// Programmatic dependent launch for the launches that follow on THIS thread (1, 0, or -1: as the process is set); returns the choice that it replaces.
+MARY_API int mary_pdl_scope(int on) {
+  const int was = t_pdl;
+  t_pdl = on < 0 ? -1 : (on ? 1 : 0);
+  return was;
+}

@@ -164,7 +164,14 @@ class Gemma4Model(nn.Module):
                     kv_heads=[max(c.layer_kv_heads(i) // self.tp.size, 1) for i in range(c.num_hidden_layers)],
                     head_dim=[c.layer_head_dim(i) for i in range(c.num_hidden_layers)])
 
+    CHAIN_MAX_ROWS = 64        # decode-sized steps: their launches are short enough that the gaps between them count
+
     def hidden(self, ids, meta, cache, soft=None):
+        plain = self.tp.size == 1 and not (self.cfg.enable_moe_block or self.cfg.hidden_size_per_layer_input)
+        with ops.chained(ids, plain and ids.shape[0] <= self.CHAIN_MAX_ROWS):
+            return self._hidden(ids, meta, cache, soft)
+
+    def _hidden(self, ids, meta, cache, soft=None):
         """Final-normed hidden states ``[T, H]`` of every row.  ``soft = (rows, embeds)`` replaces the embedding of the placeholder
         rows ``rows`` (a long tensor) by multimodal soft tokens ``embeds [len(rows), H]`` (unscaled, lm.rs:212-311); those rows take
         the pad token's per-layer embedding."""

@@ -18,6 +18,12 @@ def _k():
     return cuda
 
 
+def chained(x, on: bool = True):
+    """``with ops.chained(x):`` the launches of a decode-sized chain of dense products overlap (``ops.cuda.chained``); nothing on the CPU."""
+    import contextlib
+    return _k().chained if on and _cuda(x) else contextlib.nullcontext()
+
+
 def rmsnorm(x, weight=None, eps=1e-6):
     return _k().rmsnorm(x, weight, eps) if _cuda(x) else ref.rmsnorm(x, weight, eps)
 

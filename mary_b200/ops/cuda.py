@@ -7,6 +7,7 @@ from __future__ import annotations
 import ctypes
 import functools
 import math
+import threading
 
 import numpy as np
 import torch
@@ -208,24 +209,48 @@ def gemm_splitk(x, w, split_k: int, out=None, f32: bool = False, bias=None, swap
     return out
 
 
+class _Launch(threading.local):
+    static = 0            # depth of ``static_weights`` on this thread
+    scopes = 0            # depth of ``chained`` on this thread
+
+
+_launch = _Launch()
+declare("mary_pdl_scope", "i")
+
+
+class _Chained:
+    """While active, this thread's launches may start while their predecessor on the stream drains (programmatic dependent launch), and its GEMMs may
+    request weights ahead: for steps that are chains of small dense products.  Nothing outside the ``with`` block, and no other thread, is affected."""
+
+    def __enter__(self):
+        _launch.scopes += 1
+        if _launch.scopes == 1:
+            lib().mary_pdl_scope(1)
+
+    def __exit__(self, *exc):
+        _launch.scopes -= 1
+        if _launch.scopes == 0:
+            lib().mary_pdl_scope(-1)
+
+
+chained = _Chained()
+
+
 class _StaticWeights:
     """While active, the GEMM launchers of this thread are told that their ``w`` operand holds constant model weights, so that under
-    programmatic dependent launch (``MARY_PDL=1``) a kernel may request its first weight tiles before its predecessor has finished."""
-    depth = 0
+    programmatic dependent launch (``MARY_PDL=1``, or inside ``chained``) a kernel may request its first weight tiles before its predecessor has finished."""
 
     def __enter__(self):
         from ..utils import flags
-        if flags.get("MARY_PDL"):
-            _StaticWeights.depth += 1
-            if _StaticWeights.depth == 1:
-                lib().mary_gemm_hint_static_weights(1)
+        _launch.static += 1
+        if _launch.static == 1 and (_launch.scopes or flags.get("MARY_PDL")):
+            lib().mary_gemm_hint_static_weights(1)
 
     def __exit__(self, *exc):
         from ..utils import flags
-        if flags.get("MARY_PDL"):
-            _StaticWeights.depth -= 1
-            if _StaticWeights.depth == 0:
-                lib().mary_gemm_hint_static_weights(0)
+        _launch.static -= 1
+        if _launch.static == 0 and (_launch.scopes or flags.get("MARY_PDL")):
+            lib().mary_gemm_hint_static_weights(0)
 
 
 static_weights = _StaticWeights()

@@ -38,7 +38,7 @@ def _exact(q, k, v, table, q_lens, kv_lens, page, scale, window, cap):
 
 
 CASES = [  # D, q heads, kv heads, q_lens, kv_lens, page, window, cap
-    (256, 16, 8, [1], [1], 16, 0, 0.0), (256, 2, 1, [1, 1, 1], [777, 64, 65], 16, 0, 0.0), (256, 16, 8, [1] * 5, [1024, 1025, 1500, 31, 33], 16, 1024, 0.0),
+    (256, 16, 8, [1], [1], 16, 0, 0.0), (256, 2, 1, [1, 1, 1], [777, 64, 65], 16, 0, 0.0), (256, 16, 8, [1] * 5, [1024, 1025, 1500, 31, 33], 16, 1024, 0.0), (256, 8, 8, [2, 1], [500, 40], 16, 64, 30.0), (256, 4, 4, [1], [2049], 64, 0, 0.0),
     (256, 4, 4, [2, 4, 1], [700, 4, 129], 32, 100, 0.0), (256, 4, 1, [1, 1], [333, 2100], 64, 0, 30.0), (128, 8, 8, [1, 1], [257, 15], 16, 0, 0.0),
     (128, 8, 2, [2, 2, 1], [300, 2, 900], 16, 128, 0.0), (128, 8, 1, [1, 1], [513, 8], 16, 0, 0.0), (64, 4, 2, [1, 3], [100, 1000], 16, 0, 50.0),
     (64, 8, 1, [1], [4097], 64, 0, 0.0), (64, 4, 4, [8], [200], 16, 33, 0.0)]
@@ -51,6 +51,8 @@ def test_stream_attention(case, q8, nsplit, warps):
     from mary_b200.ops import cuda as K
     from mary_b200.runtime.kv_cache import Q8Pages
     D, Hq, Hkv, q_lens, kv_lens, page, window, cap = case
+    if not q8 and (D != 256 or max(q_lens) * Hq // Hkv > 2):
+        pytest.skip("bf16 shapes of the tensor-core kernel")
     meta, table, pages = _batch(q_lens, kv_lens, page, 1)
     g = torch.Generator(device="cuda").manual_seed(2)
     k, v = (torch.empty(pages, page, Hkv, D, dtype=torch.bfloat16, device="cuda").normal_(0.2, 1.0, generator=g) for _ in range(2))
@@ -75,10 +77,10 @@ def test_stream_attention_strided_cache():
     """Caches that are slices of a wider store (token and page strides of their own, different for K and V)."""
     from mary_b200.ops import cuda as K
     meta, table, pages = _batch([1, 1], [400, 123], 16, 3)
-    store = torch.randn(pages, 2, 16, 2, 2, 128, device="cuda").bfloat16()
+    store = torch.randn(pages, 2, 16, 2, 2, 256, device="cuda").bfloat16()
     k, v = store[:, 0, :, 0], store[:, 1, :, 1]
-    wide = torch.randn(pages, 20, 2, 128, device="cuda").bfloat16()[:, :16]
-    q = torch.randn(2, 8, 128, device="cuda").bfloat16()
+    wide = torch.randn(pages, 20, 2, 256, device="cuda").bfloat16()[:, :16]
+    q = torch.randn(2, 4, 256, device="cuda").bfloat16()
     for vc in (v, wide):
         got = K.attention_stream(q, k, vc, meta, 0.1).double()
         want = _exact(q, k.double(), vc.double(), table, [1, 1], [400, 123], 16, 0.1, 0, 0.0)
