@@ -84,7 +84,7 @@ class MLAAttention(nn.Module):
         T, H = qb.shape[0], self.H
         lat = cache.k[self.li]                                              # [pages, page, 576]
         pick, meta2 = meta.repage(64)                                       # the same for every layer of this step
-        rows = lat[pick].view(-1, 64, 576)                                  # context of every sequence in 64-token pages
+        rows = lat.index_select(0, pick).view(-1, 64, 576)                                  # context of every sequence in 64-token pages
         P, ps = rows.shape[0], 64
         if getattr(self, "_w_uk_t", None) is None:
             self._w_uk_t = self.w_uk.permute(0, 2, 1).reshape(H * 128, 512).contiguous()      # k_nope[h, n] = sum_k c_kv[k] W_UK[h, k, n]

@@ -13,6 +13,7 @@ import numpy as np
 import torch
 
 from .. import _native
+from ..utils import flags as _flags
 from ..utils.canary import empty as _empty
 
 _SIG = {
@@ -76,7 +77,8 @@ def _p(t):
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of the current stream of the current device (through ``torch.cuda.current_stream`` it costs as much host time as the launch it is for)."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 _NVTX = None
@@ -241,15 +243,13 @@ class _StaticWeights:
     programmatic dependent launch (``MARY_PDL=1``, or inside ``chained``) a kernel may request its first weight tiles before its predecessor has finished."""
 
     def __enter__(self):
-        from ..utils import flags
         _launch.static += 1
-        if _launch.static == 1 and (_launch.scopes or flags.get("MARY_PDL")):
+        if _launch.static == 1 and (_launch.scopes or _flags.get("MARY_PDL")):
             lib().mary_gemm_hint_static_weights(1)
 
     def __exit__(self, *exc):
-        from ..utils import flags
         _launch.static -= 1
-        if _launch.static == 0 and (_launch.scopes or flags.get("MARY_PDL")):
+        if _launch.static == 0 and (_launch.scopes or _flags.get("MARY_PDL")):
             lib().mary_gemm_hint_static_weights(0)
 
 
@@ -674,8 +674,8 @@ def attention_prefill(q, kcache, vcache, meta, scale, window=0, out=None, split_
     assert kcache.shape[1] == ps
     if ps in (16, 32) and meta.kv_lens_host is not None:
         pick, meta = meta.repage(64)
-        kcache = kcache[pick].view(-1, 64, Hkv, kcache.shape[3])
-        vcache = vcache[pick].view(-1, 64, Hkv, DV)
+        kcache = kcache.index_select(0, pick).view(-1, 64, Hkv, kcache.shape[3])
+        vcache = vcache.index_select(0, pick).view(-1, 64, Hkv, DV)
         ps = 64
     assert ps in (16, 64)
     blk_seq, blk_tok0, NB = _q_blocks(meta, 128, group)
