@@ -537,7 +537,7 @@ static int gemm_impl(const void* X, const void* W, void* out, int M, int N, int 
   if (batch == 1 && !g_tiles && swap < 0 && split_k == 1 &&
       (M > 128 ? (epi == EPI_STORE_BF16 || epi == EPI_STORE_F32 || (sk_epi && stream_k)) : (sk_epi && stream_k))) {
     const bool f32 = epi == EPI_STORE_F32 || epi == EPI_SK_F32;
-    PairOut o = {out, ldo, f32, glu, glu_limit, alpha, un_act, un_cols, bias, (g_static_weights && mary_pdl_enabled()) ? 1 : 0};
+    PairOut o = {out, ldo, f32, glu, glu_limit, alpha, un_act, un_cols, bias, (g_static_weights && mary_pdl_enabled()) ? 1 : 0, 0, 0};
     PairPlan plan;
     if (M > 128) {
       if (!mary_gemm_pair_plan(M, N, K, glu != 0, 256, &plan)) return MARY_ERR_BAD_ARG;

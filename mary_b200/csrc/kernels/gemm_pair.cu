@@ -49,6 +49,7 @@ struct PairParams {
   int un_act, un_cols;
   int out_f32;
   int tma_box;                            // columns per TMA store (32 or 16); 0: plain stores
+  int group, pitch;                       // group > 0 (TMA stores): output columns in groups, their starts `pitch` columns apart
   int64_t ldo;
   void* out;
   const float* bias;
@@ -325,7 +326,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
     if (lane == 0) {
       if (i0 < p.rows_r) {
         if (p.tma_box == 32) {
-          if (j0 < p.rows_c) tma_store_2d(&tm_o, smem_u32(buf), j0, i0);
+          if (j0 < p.rows_c) tma_store_2d(&tm_o, smem_u32(buf), p.group > 0 ? j0 / p.group * p.pitch + j0 % p.group : j0, i0);
         } else {
           if (j0 < p.rows_c) tma_store_2d(&tm_o, smem_u32(buf), j0, i0);
           if (c0 + 16 < (GLU ? bn / 2 : bn) && j0 + 16 < p.rows_c) tma_store_2d(&tm_o, smem_u32(buf) + 1024, j0 + 16, i0);
@@ -575,9 +576,11 @@ int mary_gemm_pair_run(const void* R, const void* C, int rows_r, int rows_c, int
   p.tma_box = 0;
   if (!swap && p.S == 1 && !o.f32 && ((uintptr_t)o.out & 15) == 0 && (o.ldo & 7) == 0 && rows_c >= 32) {
     p.tma_box = (o.glu && bn % 64) ? 16 : 32;
-    rc = store_map(&to, o.out, rows_r, rows_c, o.ldo, p.tma_box);
+    rc = store_map(&to, o.out, rows_r, o.group > 0 ? rows_c / o.group * o.pitch : rows_c, o.ldo, p.tma_box);
     if (rc) return rc;
   }
+  p.group = o.group; p.pitch = o.pitch;
+  if (o.group > 0 && (p.tma_box != 32 || o.group % 32 || rows_c % o.group || o.pitch < o.group || o.pitch % 8)) return MARY_ERR_BAD_ARG;
   if (swap) return launch<false, true>(tr, tc, to, p, clusters, stream);
   return o.glu ? launch<true, false>(tr, tc, to, p, clusters, stream) : launch<false, false>(tr, tc, to, p, clusters, stream);
 }
@@ -586,7 +589,19 @@ int mary_gemm_pair_run(const void* R, const void* C, int rows_r, int rows_c, int
 MARY_API int mary_gemm_bf16_pair(const void* X, const void* W, void* out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo, int glu, int out_f32,
                                  int bn, int splits, int swap, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || (splits != 1 && splits != 2 && splits != 4)) return MARY_ERR_BAD_ARG;
-  PairOut o = {out, ldo, out_f32, glu, 0.f, 1.0f, 0, 0, nullptr, 0};
+  PairOut o = {out, ldo, out_f32, glu, 0.f, 1.0f, 0, 0, nullptr, 0, 0, 0};
   PairPlan plan = {bn, splits};
   return swap ? mary_gemm_pair_run(W, X, N, M, K, ldw, ldx, true, o, plan, stream) : mary_gemm_pair_run(X, W, M, N, K, ldx, ldw, false, o, plan, stream);
+}
+
+// out[i, (j / group) * pitch + j % group] = X_i . W_j, bf16: the heads of a projection at a pitch of their own (group: a multiple of 32, N of group; rows of
+// ldo elements, 16-byte aligned).  The values between the groups are not written.
+MARY_API int mary_gemm_bf16_grouped_columns(const void* X, const void* W, void* out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo, int group,
+                                            int pitch, cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0 || group <= 0 || (K & 7) || (ldx & 7) || (ldw & 7)) return MARY_ERR_BAD_ARG;
+  PairOut o = {out, ldo, 0, 0, 0.f, 1.0f, 0, 0, nullptr, 0, group, pitch};
+  PairPlan plan;
+  if (!mary_gemm_pair_plan(M, N, K, false, 256, &plan)) return MARY_ERR_BAD_ARG;
+  if (plan.S > 1) plan = {128, 1};                         // the exchange of a split stores plainly
+  return mary_gemm_pair_run(X, W, M, N, K, ldx, ldw, false, o, plan, stream);
 }

@@ -14,6 +14,7 @@ struct PairOut {
   int un_act, un_cols;                   // activation of the first un_cols output features
   const float* bias;
   int w_static;
+  int group, pitch;                      // > 0: output columns in groups of `group` (a multiple of 32), `pitch` columns apart; TMA stores only
 };
 
 int mary_gemm_pair_plan(int rows_r, int rows_c, int K, bool glu, int max_bn, PairPlan* plan);

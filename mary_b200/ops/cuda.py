@@ -878,17 +878,19 @@ def gemm_batched(x, w, out, M, N, K, ldx, ldw, ldo, batch, bsx, bsw, bso):
 
 declare("mary_mla_q_rope_inplace", "pppiis")
 declare("mary_mla_fill_k_rope", "plpils")
+declare("mary_gemm_bf16_grouped_columns", "pppiiilll" + "iis")
 
 
 def mla_expand_kv(rows, w_uk_t, w_uv, H):
     """Keys and values of the expanded (non-absorbed) prefill straight into their final layout, without concatenation copies:
-    ``rows [N, 576]`` latent rows -> ``k [N, H, 192]`` (``W_UK^T c_kv`` per head by a batched GEMM over the heads that shares the
-    row operand and writes each head's 128 columns at pitch 192, then the 64 rotated dims every head shares copied behind them) and
+    ``rows [N, 576]`` latent rows -> ``k [N, H, 192]`` (``W_UK^T c_kv`` of all heads by one GEMM that
+    writes each head's 128 columns at pitch 192, then the 64 rotated dims every head shares copied behind them) and
     ``v [N, H, 128]`` (one GEMM).  ``w_uk_t [H * 128, 512]``, ``w_uv [H * 128, 512]``."""
     N = rows.shape[0]
     k = _empty(N, H, 192, dtype=torch.bfloat16, device=rows.device)
+    check(lib().mary_gemm_bf16_grouped_columns(_p(rows), _p(w_uk_t), _p(k), N, H * 128, 512, rows.stride(0), 512, H * 192, 128, 192, _stream()),
+          "gemm_bf16_grouped_columns")
     with static_weights:
-        gemm_batched(rows, w_uk_t, k, N, 128, 512, rows.stride(0), 512, H * 192, H, 0, 128 * 512, 192)
         v = gemm(rows[:, :512], w_uv)
     check(lib().mary_mla_fill_k_rope(_p(rows), rows.stride(0), _p(k), H, N, _stream()), "mla_fill_k_rope")
     return k, v.view(N, H, 128)
