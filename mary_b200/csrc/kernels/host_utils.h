@@ -15,8 +15,9 @@ int* mary_status_ptr();
 int mary_make_tmap_2d(CUtensorMap* m, const void* base, int dtype_bytes_x2, uint64_t rows, uint64_t cols, uint64_t ld,
                       uint32_t box_rows, uint32_t box_cols, int swizzle128);
 
-// 1 when the environment says MARY_PDL=1 (off by default: in CUDA-graph replay the measured step time was the same with and
-// without it, 81.2 ms against 80.1 ms at 16 sequences).
+// 1 when the launches that follow on this thread may overlap their predecessors: the process says so (MARY_PDL=1, mary_set_pdl), or the thread is in a
+// scope (mary_pdl_scope) and the process does not say no.  By default off outside of scopes: in CUDA-graph replay the K3-class step measured the same with
+// and without it, 81.2 ms against 80.1 ms at 16 sequences.
 int mary_pdl_enabled();
 
 // cudaFuncSetAttribute(MaxDynamicSharedMemorySize) applies to the CURRENT device only, so the "already raised" record is kept

@@ -97,26 +97,30 @@ int mary_ensure_dyn_smem(const void* func, size_t bytes, MarySmemSlots* slots) {
   return MARY_OK;
 }
 
-static int g_pdl = -1;          // -1: not decided yet (the environment decides at the first launch)
-
+// Programmatic dependent launch as the process is set: 1 on, 0 off, -1 nobody chose (off, but a thread's scope may turn it on), -2 not asked yet (the
+// environment is read at the first launch: "1" is on, any other value off).
+static int g_pdl = -2;
 static thread_local int t_pdl = -1;   // -1: as the process is set; else the choice of the calling thread's present scope
 
 int mary_pdl_enabled() {
-  if (t_pdl >= 0) return t_pdl;
-  if (g_pdl < 0) {
+  if (g_pdl == -2) {
     const char* e = getenv("MARY_PDL");
-    g_pdl = (e && e[0] == '1') ? 1 : 0;
+    g_pdl = (e && e[0]) ? (e[0] == '1') : -1;
   }
-  return g_pdl;
+  if (t_pdl == 0 || g_pdl == 0) return 0;              // whoever says no is heard: a step without dependent launch can always be had
+  return t_pdl == 1 || g_pdl == 1;
 }
 
 // Switch programmatic dependent launch on or off for the launches that follow (a model whose step is a chain of small dense GEMMs
-// gains from it, one with the expert pipeline in the chain loses: the caller that knows the model decides).  Graphs captured
-// before the call keep what they were captured with.
+// gains from it, one with the expert pipeline in the chain loses: the caller that knows the model decides).  Off also holds inside
+// the scopes of mary_pdl_scope.  Graphs captured before the call keep what they were captured with.
 MARY_API void mary_set_pdl(int on) { g_pdl = on ? 1 : 0; }
-// Programmatic dependent launch for the launches that follow on THIS thread (1, 0, or -1: as the process is set); returns the choice that it replaces.
+// Programmatic dependent launch for the launches that follow on THIS thread (1 unless the process is set to off, 0, or -1: as the process is set); returns
+// the choice that it replaces.
 MARY_API int mary_pdl_scope(int on) {
   const int was = t_pdl;
   t_pdl = on < 0 ? -1 : (on ? 1 : 0);
   return was;
 }
+// What the launches that follow on this thread do.
+MARY_API int mary_pdl_state() { return mary_pdl_enabled(); }

@@ -214,25 +214,28 @@ def gemm_splitk(x, w, split_k: int, out=None, f32: bool = False, bias=None, swap
 class _Launch(threading.local):
     static = 0            # depth of ``static_weights`` on this thread
     scopes = 0            # depth of ``chained`` on this thread
+    before = -1           # the thread's choice outside of it
 
 
 _launch = _Launch()
 declare("mary_pdl_scope", "i")
+declare("mary_pdl_state", "")
 
 
 class _Chained:
     """While active, this thread's launches may start while their predecessor on the stream drains (programmatic dependent launch), and its GEMMs may
-    request weights ahead: for steps that are chains of small dense products.  Nothing outside the ``with`` block, and no other thread, is affected."""
+    request weights ahead: for steps that are chains of small dense products.  Nothing outside the ``with`` block, and no other thread, is affected; a
+    process that is set to off (``MARY_PDL=0``, ``set_pdl(False)``) stays off."""
 
     def __enter__(self):
+        if _launch.scopes == 0:
+            _launch.before = lib().mary_pdl_scope(1)
         _launch.scopes += 1
-        if _launch.scopes == 1:
-            lib().mary_pdl_scope(1)
 
     def __exit__(self, *exc):
         _launch.scopes -= 1
         if _launch.scopes == 0:
-            lib().mary_pdl_scope(-1)
+            lib().mary_pdl_scope(_launch.before)
 
 
 chained = _Chained()
@@ -963,5 +966,5 @@ declare("mary_set_pdl", "i")
 
 def set_pdl(on: bool) -> None:
     """Programmatic dependent launch for the launches that follow (``MARY_PDL`` decides when nobody calls this): a gain for steps
-    that are chains of small dense GEMMs, a loss with the expert pipeline in the chain."""
+    that are chains of small dense GEMMs, a loss with the expert pipeline in the chain.  ``False`` also holds inside ``chained``."""
     lib().mary_set_pdl(int(bool(on)))
