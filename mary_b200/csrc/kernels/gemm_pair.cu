@@ -3,7 +3,7 @@
 // What bounds it.  A 128 x 256 tile of one SM moves 48 KB from L2 for every 64 columns of K, and at full tensor rate that is about 96
 // bytes a clock per SM, more than an SM can draw from L2.  Two SMs that work on one 256 x BN tile (`tcgen05.mma.cta_group::2`) hold
 // half of the column operand each: 32 KB per SM for the same arithmetic.  Shapes with few output tiles are bound by something else: one
-// tile per SM leaves SMs idle, or each of them walks a long K alone.  There a cluster of 2 or 4 pairs cuts K between the pairs and adds the
+// tile per SM leaves SMs idle, or each of them walks a long K alone.  There a cluster of 2, 4 or 8 pairs cuts K between the pairs and adds the
 // partial tiles through distributed shared memory, in a fixed order, without scratch memory and without atomics.
 //
 //   * cluster of 2 * S CTAs = S pairs; pair s multiplies the s-th part of K.  Per CTA: warp 0 issues the TMA loads of this CTA's 128
@@ -20,6 +20,8 @@
 // Measured (weights larger than L2, one-SM kernel -> this one): 8192 x 30720 x 3840 1345 -> 1235 us (1565 TFLOP/s), 8192 x 8192 x 3840 366 -> 324 us,
 // 1024 x 3840 x 65536 540 -> 375 us, 701 x 3840 x 15360 104 -> 63 us; with K split 217 x 3840 x 4096 42 -> 15 us, 384 x 2112 x 7168 23 -> 20 us,
 // 4096 x 48 x 3840 18 -> 12 us.  One tile per pair and no split, 217 x 8192 x 3840: 47 -> 20 us, 217 x 30720 x 3840: 77 -> 51 us (4.9 TB/s).
+// Narrow outputs of a long K (4 -> 8 pairs): 3 x 48 x 15360 16.6 -> 11.8 us, 16 x 128 x 7168 11.5 -> 9.2 us, 257 x 128 x 7168 11.5 -> 10.0 us.  f32 results
+// through TMA stores of 16 columns: 257 x 3840 x 256 at 256 columns 14.3 -> 10.1 us.
 #include <type_traits>
 
 #include "common.cuh"
@@ -47,8 +49,8 @@ struct PairParams {
   int act, glu_rows;                      // GLU: kind, rows between a gate row and its up row
   float glu_limit, alpha;
   int un_act, un_cols;
-  int out_f32;
-  int tma_box;                            // columns per TMA store (32 or 16); 0: plain stores
+  int tma_box;                            // columns per TMA store (32 or 16; f32: 16); 0: plain stores
+  int n_acc, acc_stride;                  // accumulators that the K blocks of a tile go round, their distance in TMEM columns
   int group, pitch;                       // group > 0 (TMA stores): output columns in groups, their starts `pitch` columns apart
   int64_t ldo;
   void* out;
@@ -117,7 +119,9 @@ __device__ __forceinline__ void tile_at(const PairParams& p, int t, int& tr, int
   }
 }
 
-template <bool GLU, bool SWAP>
+// F32: the result's type; CUT: K is cut between the pairs of a cluster (S > 1).  Each form has its own code: a launch of few blocks spends a good part of its
+// time on fetching instructions for the first time.
+template <bool GLU, bool SWAP, bool F32, bool CUT>
 __global__ void __launch_bounds__(NTHREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_c, const __grid_constant__ CUtensorMap tm_o,
                  const PairParams p) {
@@ -137,6 +141,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
   const int cluster = blockIdx.x / (2 * p.S), n_clusters = gridDim.x / (2 * p.S);
   const int total = p.tiles_r * p.tiles_c;
   const int kb0 = split * p.kb_per_split, kb1 = min(kb0 + p.kb_per_split, p.k_blocks);
+  const int n_acc = F32 ? min(p.n_acc, kb1 - kb0) : 1;                       // the last part of K may have fewer blocks than there are accumulators
 
   if (threadIdx.x < MAX_STAGES) { mbar_init(&full[threadIdx.x], 1); mbar_init(&empty[threadIdx.x], 1); }
   if (threadIdx.x >= 32 && threadIdx.x < 34) { mbar_init(&acc_full[threadIdx.x - 32], 1); mbar_init(&acc_empty[threadIdx.x - 32], 8); }
@@ -223,13 +228,17 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
         if (!mbar_wait(&acc_empty[buf], ((it >> 1) & 1) ^ 1, abort_flag, p.status, MARY_ERR_TIMEOUT_MMA)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d0 = tmem_base + buf * 256;
+        int acc = 0;
         for (int kb = kb0; kb < kb1; ++kb) {
           if (!mbar_wait(&full[stage], phase, abort_flag, p.status, MARY_ERR_TIMEOUT_TMA)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * p.stage_bytes), sb = sa + A_BYTES;
+          const uint32_t d = F32 ? d0 + acc * p.acc_stride : d0;
+          const bool begun = kb - kb0 >= n_acc;
+          if (F32 && ++acc == n_acc) acc = 0;
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            umma_f16_pair(d0, umma_desc_sw128(sa + k * 32), umma_desc_sw128(sb + k * 32), idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            umma_f16_pair(d, umma_desc_sw128(sa + k * 32), umma_desc_sw128(sb + k * 32), idesc, (begun || k > 0) ? 1u : 0u);
           umma_commit_pair(&empty[stage], mask);
           if (++stage == stages) { stage = 0; phase ^= 1; }
         }
@@ -265,7 +274,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
       for (int j = 0; j < W; ++j) {
         if (j0 + j < p.rows_c) {
           const int64_t o = (int64_t)(j0 + j) * p.ldo + i;
-          if (p.out_f32) ((float*)p.out)[o] = v[j] + b;
+          if (F32) ((float*)p.out)[o] = v[j] + b;
           else ((__nv_bfloat16*)p.out)[o] = __float2bfloat16(v[j] + b);
         }
       }
@@ -276,7 +285,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
       for (int j = 0; j < W; ++j) if (j0 + j < p.rows_c) v[j] += p.bias[j0 + j];
     }
     const int64_t o = (int64_t)i * p.ldo + j0;
-    if (p.out_f32) {
+    if (F32) {
       float* dst = (float*)p.out + o;
       if (j0 + W <= p.rows_c && ((uintptr_t)dst & 15) == 0) {
 #pragma unroll
@@ -287,9 +296,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
       }
     } else {
       __nv_bfloat16* dst = (__nv_bfloat16*)p.out + o;
-      if (j0 + W <= p.rows_c && ((uintptr_t)dst & 15) == 0) {
+      if (W % 8 == 0 && j0 + W <= p.rows_c && ((uintptr_t)dst & 15) == 0) {
 #pragma unroll
-        for (int j = 0; j < W; j += 8) {
+        for (int j = 0; j < W / 8 * 8; j += 8) {
           uint4 w;
           uint32_t* wp = (uint32_t*)&w;
 #pragma unroll
@@ -308,6 +317,26 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
   auto emit_tma = [&](int tr, int tc, int c0, const float* v) {
     const int i0 = (tr * 2 + half) * ROWS + q * 32;
     const int j0 = tc * (GLU ? bn / 2 : bn) + c0;
+    if constexpr (F32) {
+      // f32: the 32 columns in two boxes of 16, rows of 64 bytes in the 64-byte swizzle
+#pragma unroll
+      for (int h = 0; h < 2; ++h, ++n_stored) {
+        uint8_t* buf = stage_out + (n_stored & 1) * 2048;
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          *(float4*)(buf + lane * 64 + ((c ^ ((lane >> 1) & 3)) << 4)) =
+              make_float4(v[16 * h + 4 * c], v[16 * h + 4 * c + 1], v[16 * h + 4 * c + 2], v[16 * h + 4 * c + 3]);
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+          if (i0 < p.rows_r && j0 + 16 * h < p.rows_c && c0 + 16 * h < (GLU ? bn / 2 : bn)) tma_store_2d(&tm_o, smem_u32(buf), j0 + 16 * h, i0);
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+      }
+      return;
+    }
     uint8_t* buf = stage_out + (n_stored & 1) * 2048;
     if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");      // the store before last has read this buffer
     __syncwarp();
@@ -336,6 +365,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
     }
     ++n_stored;
   };
+  // 32 columns of this thread's row: the sum of the tile's accumulators, in a fixed order
+  auto read32 = [&](uint32_t at, uint32_t* r) {
+    tmem_ld_32x32b_x32(at, r);
+    tmem_ld_wait();
+    if constexpr (!F32) return;
+    for (int a = 1; a < n_acc; ++a) {
+      uint32_t t[32];
+      tmem_ld_32x32b_x32(at + a * p.acc_stride, t);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __uint_as_float(t[j]));
+    }
+  };
   if (warp >= 2) {
     pdl_wait();                            // before the first store: an earlier kernel may still read what this one overwrites
     const uint32_t empty0 = mapa(smem_u32(acc_empty), rank & ~1u);
@@ -345,22 +387,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
       if (!mbar_wait(&acc_full[buf], (it >> 1) & 1, abort_flag, p.status, MARY_ERR_TIMEOUT_MMA)) { ok = false; break; }
       tc_fence_after();
       const uint32_t taddr = tmem_base + buf * 256 + ((uint32_t)(q * 32) << 16);
-      if (p.S == 1) {
+      if constexpr (!CUT) {
         int tr, tc;
         tile_at(p, t, tr, tc);
 #pragma unroll 1
         for (int c0 = 0; c0 < (GLU ? bn / 2 : bn); c0 += 32) {
           uint32_t r[32];
           float v[32];
-          tmem_ld_32x32b_x32(taddr + c0, r);
           if (GLU) {
             uint32_t u[32];
+            tmem_ld_32x32b_x32(taddr + c0, r);
             tmem_ld_32x32b_x32(taddr + bn / 2 + c0, u);
             tmem_ld_wait();
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = glu_f(p.act, __uint_as_float(r[j]) * p.alpha, __uint_as_float(u[j]) * p.alpha, p.glu_limit);
           } else {
-            tmem_ld_wait();
+            read32(taddr + c0, r);
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(r[j]) * p.alpha;
           }
@@ -385,8 +427,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
 #pragma unroll 1
         for (int c0 = 0; c0 < bn; c0 += 32) {
           uint32_t r[32];
-          tmem_ld_32x32b_x32(taddr + c0, r);
-          tmem_ld_wait();
+          read32(taddr + c0, r);
 #pragma unroll
           for (int j = 0; j < 8; ++j) part[(c0 / 4 + j) * ROWS + row] = make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]);
         }
@@ -394,12 +435,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
     }
   }
   __syncwarp();
-  if (p.S > 1) {
+  if constexpr (CUT) {
     cluster_sync_all();                    // every partial tile of the cluster is in shared memory
     if (warp >= 2 && ok && cluster < total && !*abort_flag) {
       int tr, tc;
       tile_at(p, cluster, tr, tc);
-      const int share = (GLU ? bn / 2 : bn) / p.S;        // columns that this CTA finishes: a multiple of 8
+      const int share = (GLU ? bn / 2 : bn) / p.S;        // columns that this CTA finishes: a multiple of 8, or of 4 with 8 pairs
       const uint32_t mine = smem_u32(smem) + row * 16;
       // W columns at a time, all pairs' values of them requested before the first is used
       auto gather = [&](auto width, auto pairs, int c0) {
@@ -434,15 +475,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
         int c = 0;
         for (; c + 16 <= share; c += 16) gather(std::integral_constant<int, 16>{}, std::integral_constant<int, 2>{}, first + c);
         if (c < share) gather(std::integral_constant<int, 8>{}, std::integral_constant<int, 2>{}, first + c);
-      } else {
+      } else if (p.S == 4) {
         int c = 0;
         for (; c + 16 <= share; c += 16) gather(std::integral_constant<int, 16>{}, std::integral_constant<int, 4>{}, first + c);
         if (c < share) gather(std::integral_constant<int, 8>{}, std::integral_constant<int, 4>{}, first + c);
+      } else if constexpr (!GLU) {
+        int c = 0;
+        for (; c + 8 <= share; c += 8) gather(std::integral_constant<int, 8>{}, std::integral_constant<int, 8>{}, first + c);
+        if (c < share) gather(std::integral_constant<int, 4>{}, std::integral_constant<int, 8>{}, first + c);
       }
     }
     __syncwarp();
   }
-  if (warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");    // the stores are complete
+  if (!CUT && warp >= 2 && lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");    // the stores are complete
   __syncwarp();
   tc_fence_before();
   cluster_sync_all();                      // neither shared memory nor TMEM goes while the other CTAs may still reach it
@@ -452,10 +497,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_r, const __grid_constant
   }
 }
 
-template <bool GLU, bool SWAP>
+template <bool GLU, bool SWAP, bool F32, bool CUT>
 int launch(const CUtensorMap& tr, const CUtensorMap& tc, const CUtensorMap& to, const PairParams& p, int clusters, cudaStream_t stream) {
   static MarySmemSlots smem_set = {};
-  if (int rc = mary_ensure_dyn_smem((const void*)gemm_pair_kernel<GLU, SWAP>, SMEM, &smem_set)) return rc;
+  if (int rc = mary_ensure_dyn_smem((const void*)gemm_pair_kernel<GLU, SWAP, F32, CUT>, SMEM, &smem_set)) return rc;
+  if (p.S > 4 && cudaFuncSetAttribute(gemm_pair_kernel<GLU, SWAP, F32, CUT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return MARY_ERR_CUDA;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(clusters * 2 * p.S);
   cfg.blockDim = dim3(NTHREADS);
@@ -469,20 +515,20 @@ int launch(const CUtensorMap& tr, const CUtensorMap& tc, const CUtensorMap& to, 
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = mary_pdl_enabled() ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, gemm_pair_kernel<GLU, SWAP>, tr, tc, to, p) != cudaSuccess) return MARY_ERR_CUDA;
+  if (cudaLaunchKernelEx(&cfg, gemm_pair_kernel<GLU, SWAP, F32, CUT>, tr, tc, to, p) != cudaSuccess) return MARY_ERR_CUDA;
   MARY_CHECK_LAUNCH();
   return MARY_OK;
 }
 
-// bf16 output rows in boxes of 32 rows x `box` columns
-int store_map(CUtensorMap* m, void* out, int rows, int cols, int64_t ld, int box) {
+// output rows in boxes of 32 rows x `box` columns
+int store_map(CUtensorMap* m, void* out, int f32, int rows, int cols, int64_t ld, int box) {
   PFN_encodeTiled enc = mary_encode_fn();
   if (!enc) return MARY_ERR_CUDA;
   cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
   cuuint32_t boxes[2] = {(cuuint32_t)box, 32}, estr[2] = {1, 1};
-  CUresult r = enc(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, out, dims, strides, boxes, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   box == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+  CUresult r = enc(m, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, out, dims, strides, boxes, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   box * (f32 ? 4 : 2) == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? MARY_OK : MARY_ERR_CUDA;
 }
@@ -490,14 +536,20 @@ int store_map(CUtensorMap* m, void* out, int rows, int cols, int64_t ld, int box
 }  // namespace
 
 // Clusters of 2 S CTAs that the current device runs at a time: clusters of 4 and 8 leave some SMs of a processor cluster without a partner.
+// Clusters of 16 are beyond what every device promises: 0 where there are none.
 static int resident_clusters(int S) {
-  static int known[MARY_MAX_DEVICES][3];                   // 0: not asked yet
+  static int known[MARY_MAX_DEVICES][4];                   // 0: not asked yet, -1: none
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MARY_MAX_DEVICES) return 1;
-  int& n = known[dev][S == 1 ? 0 : (S == 2 ? 1 : 2)];
-  if (n) return n;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MARY_MAX_DEVICES) return S == 8 ? 0 : 1;
+  int& n = known[dev][S == 1 ? 0 : (S == 2 ? 1 : (S == 4 ? 2 : 3))];
+  if (n) return n > 0 ? n : 0;
   static MarySmemSlots smem_set = {};
-  if (mary_ensure_dyn_smem((const void*)gemm_pair_kernel<false, false>, SMEM, &smem_set)) return 1;
+  if (mary_ensure_dyn_smem((const void*)gemm_pair_kernel<false, false, false, true>, SMEM, &smem_set)) return S == 8 ? 0 : 1;
+  if (S == 8 && cudaFuncSetAttribute(gemm_pair_kernel<false, false, false, true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    n = -1;
+    return 0;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(mary_num_sms() / (2 * S) * (2 * S));
   cfg.blockDim = dim3(NTHREADS);
@@ -509,15 +561,16 @@ static int resident_clusters(int S) {
   cfg.attrs = at;
   cfg.numAttrs = 1;
   int got = 0;
-  if (cudaOccupancyMaxActiveClusters(&got, gemm_pair_kernel<false, false>, &cfg) != cudaSuccess || got < 1) { cudaGetLastError(); got = 1; }
+  if (cudaOccupancyMaxActiveClusters(&got, gemm_pair_kernel<false, false, false, true>, &cfg) != cudaSuccess || got < 1) { cudaGetLastError(); got = S == 8 ? -1 : 1; }
   n = got;
-  return got;
+  return got > 0 ? got : 0;
 }
 
-// Width (32 .. max_bn) and K split with the smallest estimated time, in ns.  Measured between 1 and 701 rows: a K block of 64 takes 1.08 ns per column
-// of the tile (the MMAs) and at least 172; with every SM busy the 16 KB + 64 BN bytes that an SM draws for it arrive at 110 GB/s; storing a tile that
-// no next tile hides takes 6 ns per column, and an exchange of partial sums 0.5 us + 6.5 ns per column and pair; memory gives 6.2 TB/s to all SMs and a
-// quarter less to few of them.
+// Width (32 .. max_bn) and K split with the smallest estimated time, in ns.  Measured: a K block of 64 takes 1.08 ns per column of the tile (the MMAs) and
+// at least 172; with every SM busy the 16 KB + 64 BN bytes that an SM draws for it arrive at 110 GB/s; storing a tile takes 6 ns per column (16 with
+// the GLU's exponentials) where no next tile hides it, and never less than that + 0.4 us per tile; an exchange of partial sums 0.5 us + 6.5 ns per
+// column and pair (3.6 with 8 pairs, which read more of it at a time); memory gives 6.2 TB/s to all SMs and a quarter less to few of them.  Over 700
+// shapes of 3 to 8192 rows, 16 to 3840 outputs and K of 128 to 15360 the choice takes 1.1 % longer on average than the fastest of all widths and splits.
 int mary_gemm_pair_plan(int rows_r, int rows_c, int K, bool glu, int max_bn, PairPlan* plan) {
   const int sms = mary_num_sms();
   const int kb = (K + BK - 1) / BK;
@@ -527,17 +580,18 @@ int mary_gemm_pair_plan(int rows_r, int rows_c, int K, bool glu, int max_bn, Pai
   for (int bn = max_bn; bn >= 32; bn -= 32) {
     if (glu && bn < 64) continue;
     const int64_t tc = (rows_c + (glu ? bn / 2 : bn) - 1) / (glu ? bn / 2 : bn);
-    for (int S = 1; S <= 4; S *= 2) {
+    for (int S = 1; S <= 8; S *= 2) {
       if (S > 1 && kb < 4 * S) continue;
+      if (S > 4 && glu) continue;
       if (glu && bn % (16 * S)) continue;                  // every CTA of the cluster finishes a multiple of 8 outputs
       if (((kb + S - 1) / S) * (S - 1) >= kb) continue;
       const int64_t slots = resident_clusters(S), tiles = tr * tc;
       if (S > 1 && tiles > slots) continue;                // more tiles than clusters: the exchange would not overlap anything
       const int64_t waves = (tiles + slots - 1) / slots;
       const double busy = (double)(tiles < slots ? tiles : slots) * 2 * S / sms;
-      const double per = fmax(fmax(1.08 * bn, 172.0), busy * (A_BYTES + bn * 64) / 110.0);
-      double t = fmax((double)waves * ((kb + S - 1) / S) * per, memory * (1.25 - 0.25 * busy));
-      t += S > 1 ? 500.0 + 6.5 * bn * S : 6.0 * bn;
+      const double per = fmax(fmax(1.08 * bn, 172.0), busy * (A_BYTES + bn * 64) / 110.0), store = (glu ? 16.0 : 6.0) * bn;
+      double t = fmax((double)waves * fmax(((kb + S - 1) / S) * per, waves > 1 ? store + 390.0 : 0.0), memory * (1.25 - 0.25 * busy));
+      t += S > 1 ? 500.0 + (S == 8 ? 3.6 : 6.5) * bn * S : store;
       if (best == 0 || t < best) { best = t; plan->bn = bn; plan->S = S; }
     }
   }
@@ -554,7 +608,7 @@ int mary_gemm_pair_run(const void* R, const void* C, int rows_r, int rows_c, int
   p.tiles_c = (rows_c + (o.glu ? bn / 2 : bn) - 1) / (o.glu ? bn / 2 : bn);
   p.k_blocks = (K + BK - 1) / BK;
   p.kb_per_split = (p.k_blocks + p.S - 1) / p.S;
-  if (bn % 32 || bn < 32 || bn > 256 || (o.glu && (swap || bn < 64 || bn % (16 * p.S))) || p.kb_per_split * (p.S - 1) >= p.k_blocks) return MARY_ERR_BAD_ARG;
+  if (bn % 32 || bn < 32 || bn > 256 || (o.glu && (swap || bn < 64 || p.S > 4 || bn % (16 * p.S))) || p.kb_per_split * (p.S - 1) >= p.k_blocks) return MARY_ERR_BAD_ARG;
   p.stage_bytes = A_BYTES + bn * BK;                       // BN / 2 rows of 128 bytes
   p.stages = RING / p.stage_bytes;
   if (p.stages > MAX_STAGES) p.stages = MAX_STAGES;
@@ -562,11 +616,26 @@ int mary_gemm_pair_run(const void* R, const void* C, int rows_r, int rows_c, int
   p.act = o.glu ? o.glu - 1 : 0; p.glu_rows = rows_c;
   p.glu_limit = o.glu_limit; p.alpha = o.alpha;
   p.un_act = o.un_act; p.un_cols = o.un_cols;
-  p.out_f32 = o.f32; p.ldo = o.ldo; p.out = o.out; p.bias = o.bias;
+  p.ldo = o.ldo; p.out = o.out; p.bias = o.bias;
   p.w_static = o.w_static; p.status = mary_status_ptr();
   const int total = p.tiles_r * p.tiles_c;
   const int slots = mary_num_sms() / 2;
   const int clusters = p.S > 1 ? total : (total < slots ? total : slots);
+  // f32 results: the tensor core cuts off what an addition of 16 products leaves below the accumulator's last place, always downwards, so the error
+  // grows with the length of a chain.  TMEM columns that the tile leaves free take further accumulators, until no chain is longer than the one-SM kernel's
+  // dealing of K among all SMs makes it (at most 16 parts, at least 4 blocks), 3 x 128 x 7168: relative error 1.9e-6 -> 4e-7.
+  p.acc_stride = bn <= 32 ? 32 : (bn <= 64 ? 64 : (bn <= 128 ? 128 : 256));
+  p.n_acc = 1;
+  if (o.f32 && !o.glu) {
+    const int sms = mary_num_sms(), fit = (total <= clusters ? 512 : 256) / p.acc_stride;
+    const int m = swap ? rows_c : rows_r, n = swap ? rows_r : rows_c;
+    const int64_t tiles = m <= 256 ? (n + 127) / 128 : (int64_t)((m + 127) / 128) * ((n + 63) / 64);
+    int chain = (int)((tiles * p.k_blocks + sms - 1) / sms);
+    if (chain < (p.k_blocks + 15) / 16) chain = (p.k_blocks + 15) / 16;
+    if (chain < 4) chain = 4;
+    const int want = (p.kb_per_split + chain - 1) / chain;
+    p.n_acc = want < fit ? want : fit;
+  }
   CUtensorMap tr, tc;
   int rc = mary_make_tmap_2d(&tr, R, 4, rows_r, K, ldr, ROWS, BK, 1);
   if (rc) return rc;
@@ -574,21 +643,28 @@ int mary_gemm_pair_run(const void* R, const void* C, int rows_r, int rows_c, int
   if (rc) return rc;
   CUtensorMap to = tr;                                     // only read when tma_box is set
   p.tma_box = 0;
-  if (!swap && p.S == 1 && !o.f32 && ((uintptr_t)o.out & 15) == 0 && (o.ldo & 7) == 0 && rows_c >= 32) {
-    p.tma_box = (o.glu && bn % 64) ? 16 : 32;
-    rc = store_map(&to, o.out, rows_r, o.group > 0 ? rows_c / o.group * o.pitch : rows_c, o.ldo, p.tma_box);
+  if (!swap && p.S == 1 && ((uintptr_t)o.out & 15) == 0 && (o.ldo & (o.f32 ? 3 : 7)) == 0 && rows_c >= 32) {
+    p.tma_box = (o.f32 || (o.glu && bn % 64)) ? 16 : 32;
+    rc = store_map(&to, o.out, o.f32, rows_r, o.group > 0 ? rows_c / o.group * o.pitch : rows_c, o.ldo, p.tma_box);
     if (rc) return rc;
   }
   p.group = o.group; p.pitch = o.pitch;
   if (o.group > 0 && (p.tma_box != 32 || o.group % 32 || rows_c % o.group || o.pitch < o.group || o.pitch % 8)) return MARY_ERR_BAD_ARG;
-  if (swap) return launch<false, true>(tr, tc, to, p, clusters, stream);
-  return o.glu ? launch<true, false>(tr, tc, to, p, clusters, stream) : launch<false, false>(tr, tc, to, p, clusters, stream);
+  auto go = [&](auto glu, auto sw, auto f32) {
+    return p.S > 1 ? launch<glu, sw, f32, true>(tr, tc, to, p, clusters, stream) : launch<glu, sw, f32, false>(tr, tc, to, p, clusters, stream);
+  };
+  const std::true_type yes;
+  const std::false_type no;
+  if (o.glu) return o.f32 ? go(yes, no, yes) : go(yes, no, no);
+  if (swap) return o.f32 ? go(no, yes, yes) : go(no, yes, no);
+  return o.f32 ? go(no, no, yes) : go(no, no, no);
 }
 
 // The kernel with a given width (a multiple of 32) and K split; swap as in mary_gemm_bf16.  glu: 0, or 1 + kind.
 MARY_API int mary_gemm_bf16_pair(const void* X, const void* W, void* out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo, int glu, int out_f32,
                                  int bn, int splits, int swap, cudaStream_t stream) {
-  if (M <= 0 || N <= 0 || K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || (splits != 1 && splits != 2 && splits != 4)) return MARY_ERR_BAD_ARG;
+  if (M <= 0 || N <= 0 || K <= 0 || (K & 7) || (ldx & 7) || (ldw & 7) || (splits != 1 && splits != 2 && splits != 4 && splits != 8)) return MARY_ERR_BAD_ARG;
+  if (splits == 8 && resident_clusters(8) < 1) return MARY_ERR_BAD_ARG;
   PairOut o = {out, ldo, out_f32, glu, 0.f, 1.0f, 0, 0, nullptr, 0, 0, 0};
   PairPlan plan = {bn, splits};
   return swap ? mary_gemm_pair_run(W, X, N, M, K, ldw, ldx, true, o, plan, stream) : mary_gemm_pair_run(X, W, M, N, K, ldx, ldw, false, o, plan, stream);

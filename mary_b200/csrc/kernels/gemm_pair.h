@@ -3,7 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-struct PairPlan { int bn, S; };          // tile width (multiple of 32), pairs that share K (1, 2 or 4)
+struct PairPlan { int bn, S; };          // tile width (multiple of 32), pairs that share K (1, 2, 4 or 8)
 
 struct PairOut {
   void* out;

@@ -163,7 +163,8 @@ declare("mary_gemm_bf16_pair", "pppiiilll" + "iiiiis")
 
 
 def gemm_pair(x, w, bn: int, splits: int = 1, swap: bool = False, glu: str | None = None, f32: bool = False):
-    """The two-SM GEMM with a given tile width and K split (the launchers choose both by themselves)."""
+    """The two-SM GEMM with a given tile width and K split (the launchers choose both by themselves): ``bn`` a multiple of 32 up to 256, ``splits`` 1, 2 or
+    4 (with ``glu`` such that every CTA of a cluster finishes 8 outputs), 8 without ``glu`` where the device runs clusters of 16."""
     _bf16(x), _bf16(w)
     M, K = x.shape
     N = w.shape[0] // (2 if glu else 1)

@@ -71,3 +71,76 @@ def test_pair_bias_views_and_activation(M, N, K):
     _close(out[:, 1:1 + N], want, K)
     assert not out[:, 0].any() and not out[:, 1 + N:].any()
     assert K_.last_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(3, 128, 7168), (33, 384, 4096), (100, 96, 15360), (217, 3840, 4096), (300, 128, 7168), (16, 1536, 15360)])
+def test_f32_sums_are_as_exact_as_sixteen_slices(M, N, K):
+    """Router logits and partial sums: an addition in the tensor core loses half a unit (2^-24 of the sum so far) on average, always downwards.  A sum
+    that grows to its value over K / 16 / 16 additions therefore loses half of that many units at most; the f32 additions of the slices lose less than 8."""
+    from mary_b200.ops import cuda as K_
+    x, w = _problem(M, N, K, seed=3)
+    want = x.double() @ w.double().t()
+    err = (K_.linear_f32(x, w).double() - want).norm() / want.norm()
+    assert err < (K / 16 / 16 / 2 + 8) * 2.0 ** -24, err
+
+
+@pytest.mark.parametrize("M", [1, 3, 33, 100, 128])
+@pytest.mark.parametrize("N,K", [(1100, 4096), (40, 2568), (2112, 7168), (129, 15360), (384, 3840)])
+def test_few_rows(M, N, K):
+    """Products of at most 128 rows whose K is cut: the weights are the row operand."""
+    from mary_b200.ops import cuda as K_
+    x, w = _problem(M, N, K, seed=M)
+    want = x.double() @ w.double().t()
+    for f in (K_.linear, K_.linear_f32):
+        got = f(x, w)
+        _close(got, want, K)
+        assert torch.equal(got, f(x, w))
+    bias = torch.randn(N, device="cuda")
+    _close(K_.linear(x, w, bias), want + bias.double(), K)
+    cols = N - 13
+    acted = want.clone()
+    acted[:, :cols] = torch.nn.functional.silu(want[:, :cols])
+    _close(K_.linear_act(x, w, "silu", cols), acted, K)
+    assert K_.last_status() == 0
+
+
+@pytest.mark.parametrize("bn", [32, 64, 96, 224, 256])
+@pytest.mark.parametrize("splits", [1, 2, 4, 8])
+@pytest.mark.parametrize("swap", [False, True])
+def test_every_width_and_split(bn, splits, swap):
+    """Widths, splits (also a last part of K of one block, and a last block that is cut) and both operand orders, at sizes that leave partial tiles."""
+    from mary_b200.ops import cuda as K_
+    for M, N, K in ((70, 300, 64 * (5 * (splits - 1) + 1)), (300, 264, 64 * 9 * splits - 24)):
+        x, w = _problem(M, N, K, seed=bn + splits)
+        want = x.double() @ w.double().t()
+        for f32 in (False, True):
+            _close(K_.gemm_pair(x, w, bn, splits, swap=swap, f32=f32), want, K)
+    assert K_.last_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 128, 15360), (300, 40, 7168), (129, 33, 2112), (70, 3840, 256), (2050, 1032, 136)])
+def test_f32_rows(M, N, K):
+    """f32 results: clusters of 16, stores of 16 columns, rows that end inside a box or that no 16-byte store can take, a bias."""
+    from mary_b200.ops import cuda as K_
+    x, w = _problem(M, N, K, seed=7)
+    want = x.double() @ w.double().t()
+    for pad in (0, 4, 3):
+        out = torch.zeros(M, N + pad, device="cuda")
+        K_.gemm(x, w, out=out[:, :N], epi="f32")
+        _close(out[:, :N], want, K)
+        assert not out[:, N:].any()
+    bias = torch.randn(N, device="cuda")
+    _close(K_.gemm(x, w, bias=bias, epi="f32"), want + bias.double(), K)
+    assert K_.last_status() == 0
+
+
+@pytest.mark.parametrize("bn", [64, 96, 224, 256])
+@pytest.mark.parametrize("splits", [1, 2, 4])
+def test_every_width_and_split_of_glu(bn, splits):
+    from mary_b200.ops import cuda as K_
+    if bn % (16 * splits):
+        pytest.skip("columns of a CTA")
+    x, w = _problem(300, 2 * 264, 2112, seed=bn)
+    gu = x.double() @ w.double().t()
+    _close(K_.gemm_pair(x, w, bn, splits, glu="swiglu"), torch.nn.functional.silu(gu[:, :264]) * gu[:, 264:], 2112)
+    assert K_.last_status() == 0
