@@ -519,6 +519,16 @@ MARY_API int mary_gemm_bf16_rs(const void* X, const void* W, int M, int N, int K
                    rows_per_rank, stream);
 }
 
+// Whether a product of more than 256 rows stays on the one-SM kernel: it starts and ends a microsecond sooner than clusters do, which counts where one
+// wave of its smallest tiles does all the work and K is short, unless the tiles are so few that cutting K is worth more.  us, one-SM / two-SM: 701 x 512 x
+// 512 6.2 / 7.1, 1024 x 512 x 1024 7.5 / 8.7, 701 x 1024 x 2048 10.1 / 11.0, 8192 x 128 x 3072 12.8 / 15.2; 257 x 96 x 1024 (few tiles) 8.2 / 7.4,
+// 1024 x 1024 x 4096 (long K) 15.7 / 15.1.
+static bool one_sm_wins(int M, int N, int K) {
+  const int sms = mary_num_sms(), kb = (K + BK - 1) / BK, tr = (M + BM - 1) / BM;
+  const int64_t tiles = (int64_t)tr * ((N + 63) / 64);
+  return M > 256 && tiles <= sms && kb <= 48 && (kb <= 8 || 2 * tiles > (kb > 32 ? 5 : 3) * kb);
+}
+
 static int gemm_impl(const void* X, const void* W, void* out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo, int batch,
                      int64_t bsx, int64_t bsw, int64_t bso, const float* bias, float alpha, int glu, int epi, int split_k, int swap,
                      const uint64_t* rs_bufs, int rs_world, int rs_src, int rs_rpr, cudaStream_t stream, float* ws, int64_t ws_floats,
@@ -534,7 +544,7 @@ static int gemm_impl(const void* X, const void* W, void* out, int M, int N, int 
   // The two-SM kernel (gemm_pair.cu) takes plain products of more rows than one 128-row tile, with the GLU in its epilogue, and, with the weights
   // as the row operand, the products of fewer rows whose K is to be cut so that every SM works: 15.5 against 18.0 us at 1 x 8192 x 3840, 24.2
   // against 25.6 us at 1 x 3840 x 15360, 28.0 against 34.5 us at 100 x 3840 x 15360.
-  if (batch == 1 && !g_tiles && swap < 0 && split_k == 1 &&
+  if (batch == 1 && !g_tiles && swap < 0 && split_k == 1 && (glu || sk_epi || !one_sm_wins(M, N, K)) &&
       (M > 128 ? (epi == EPI_STORE_BF16 || epi == EPI_STORE_F32 || (sk_epi && stream_k)) : (sk_epi && stream_k))) {
     const bool f32 = epi == EPI_STORE_F32 || epi == EPI_SK_F32;
     PairOut o = {out, ldo, f32, glu, glu_limit, alpha, un_act, un_cols, bias, (g_static_weights && mary_pdl_enabled()) ? 1 : 0, 0, 0};
@@ -547,8 +557,7 @@ static int gemm_impl(const void* X, const void* W, void* out, int M, int N, int 
     return mary_gemm_pair_run(W, X, N, M, K, ldw, ldx, true, o, plan, stream);
   }
   const bool use_swap = glu ? true : (swap < 0 ? (M <= 256) : swap != 0);
-  // GLU without swap would need the weight operand on the column side; for large M the host falls back to
-  // a plain GEMM followed by the GLU kernel, so here GLU implies swap.
+  // GLU without swap would need the weight operand on the column side, so here GLU implies swap.
   GemmParams p;
   p.K = K;
   p.k_blocks = (K + BK - 1) / BK;

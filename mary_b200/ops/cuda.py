@@ -329,14 +329,25 @@ def linear_act(x, w, act: str, cols: int):
     return out
 
 
+# With a short K the exponentials of a large GLU epilogue (16 ns per column of gate and up) take longer than the main loop that should hide them, and four warps
+# of an SM do them: there a launch of its own, which uses every warp, is the faster form.  us, fused / two launches: 8192 x 1024 x 1024 48 / 37, 257 x 8192 x
+# 1024 29 / 22, 4096 x 512 x 1024 18 / 16; 1024 x 512 x 1024 9.9 / 10.7 (too few outputs), 2048 x 1536 x 4096 41.2 / 41.7 (long K).
+GLU_SPLIT_MAX_K = 1536
+GLU_SPLIT_MIN_OUTPUTS = 1 << 20
+
+
 def linear_glu(x, w_gu, act: str = "geglu", limit: float = 0.0, out=None):
     """``out``: a row view that receives the result (its rows 16-byte aligned where the product is)."""
-    M = x.shape[0]
+    M, F = x.shape[0], w_gu.shape[0] // 2
     if x.dtype == torch.float32 or x.shape[1] % 8 or w_gu.shape[0] % 16:
         from .cuda_hybrid import glu_any
         y = glu_any(linear(x, w_gu), act, limit)
     elif M == 1 and act in ("geglu", "swiglu", "clamped") and x.shape[1] <= 8192 and w_gu.numel() * 2 <= MATVEC_GLU_MAX_BYTES and w_gu.stride(0) % 8 == 0:
         return step_matvec(x, w_gu, mode=act, alpha=limit if act == "clamped" else 1.0, out=out)
+    elif (M > 256 and x.shape[1] <= GLU_SPLIT_MAX_K and M * F >= GLU_SPLIT_MIN_OUTPUTS
+          and (out is None or (out.data_ptr() % 16 == 0 and out.stride(0) % 8 == 0))):       # rows that the GLU kernel stores
+        with static_weights:
+            y = glu(gemm(x, w_gu), act, limit, out)
     else:
         with static_weights:
             return gemm(x, w_gu, out=out, glu=act, limit=limit)

@@ -144,3 +144,32 @@ def test_every_width_and_split_of_glu(bn, splits):
     gu = x.double() @ w.double().t()
     _close(K_.gemm_pair(x, w, bn, splits, glu="swiglu"), torch.nn.functional.silu(gu[:, :264]) * gu[:, 264:], 2112)
     assert K_.last_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K", [(257, 64, 8), (300, 1000, 1024), (384, 2112, 2048), (701, 512, 512), (8192, 128, 3072), (1024, 1024, 3080), (257, 96, 1024)])
+def test_short_products_of_many_rows(M, N, K):
+    """Around the line between the one-SM and the two-SM kernel (tiles of one wave, K blocks against tiles)."""
+    from mary_b200.ops import cuda as K_
+    x, w = _problem(M, N, K, seed=5)
+    want = x.double() @ w.double().t()
+    for f in (K_.linear, K_.linear_f32):
+        _close(f(x, w), want, K)
+        assert torch.equal(f(x, w), f(x, w))
+    assert K_.last_status() == 0
+
+
+@pytest.mark.parametrize("M,F,K,two", [(257, 8192, 1024, True), (2048, 512, 1536, True), (2048, 512, 1544, False), (2040, 512, 1024, False), (256, 8192, 1024, False)])
+@pytest.mark.parametrize("act", ["geglu", "swiglu", "situ"])
+def test_short_glu_products_take_two_launches(M, F, K, two, act):
+    from mary_b200.ops import cuda as K_
+    x, w = _problem(M, 2 * F, K, seed=11)
+    got, parts = K_.linear_glu(x, w, act), K_.glu(K_.gemm(x, w), act)
+    assert torch.equal(got, parts) == two                                              # fused, gate and up are not rounded to bf16 in between
+    assert (got.double() - parts.double()).norm() / parts.double().norm() < 2.0 ** -7   # two more roundings of 2^-9
+    out = torch.zeros(M, F + 24, dtype=torch.bfloat16, device="cuda")
+    K_.linear_glu(x, w, act, out=out[:, 8:8 + F])
+    assert torch.equal(out[:, 8:8 + F], got) and not out[:, :8].any() and not out[:, 8 + F:].any()
+    out.zero_()
+    K_.linear_glu(x, w, act, out=out[:, 1:1 + F])                                      # rows that no 16-byte store can take
+    assert (out[:, 1:1 + F].double() - got.double()).norm() / got.double().norm() < 2.0 ** -7 and not out[:, 0].any() and not out[:, 1 + F:].any()
+    assert K_.last_status() == 0
