@@ -507,8 +507,8 @@ __global__ void __launch_bounds__(1024) softcap_ce_kernel(__nv_bfloat16* __restr
   }
 }
 
-// The same with the row kept in shared memory by a cluster, whose CTAs hold neighbouring parts of it: the logits are read once and written once, and
-// three CTAs of an SM overlap their loads, arithmetic and stores.  A value costs one exponential per pass: tanh is its series x (1 - x^2 / 3 + ..) to
+// The same for a cap > 0, with the row kept in shared memory by a cluster, whose CTAs hold neighbouring parts of it: the logits are read once and written
+// once, and two or three CTAs of an SM overlap their loads, arithmetic and stores.  A value costs one exponential per pass: tanh is its series x (1 - x^2 / 3 + ..) to
 // x^13 (relative error below 1e-8 up to 0.35) in packed pairs, the exponential form only for vectors with a larger argument; and with 0 < cap <= 40 the
 // cap itself is the reference of the sum, which needs no running maximum (exp(-2 cap) stays a normal number).  The form above reads the row twice from
 // memory and takes six special-function results per value: 533 us for 1024 rows of 262144, this form 437 us.
@@ -560,17 +560,19 @@ softcap_ce_cluster_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const 
   const int64_t row = blockIdx.y;
   __nv_bfloat16* const lr = logits + row * ld;
   const int lo = min(V, rank * part), n = min(V, lo + part) - lo;                  // a multiple of 8
-  const float inv_cap = cap > 0.f ? 1.f / cap : 0.f;
+  const float inv_cap = 1.f / cap;
   const int64_t lab = labels[row];
   const bool counted = lab >= 0 && lab < V;                                        // a label outside the vocabulary: the row is ignored
   const int label = counted ? (int)lab - lo : -1;
-  const bool fixed = cap > 0.f && cap <= 40.f;
+  const bool fixed = cap <= 40.f;
   const __nv_bfloat162 edge = __bfloat162bfloat162(__float2bfloat16_rd(0.35f * cap));
   constexpr float LOG2E = 1.4426950408889634f;
-  const float slope = (cap > 0.f ? cap : 1.f) * LOG2E;
+  const float slope = cap * LOG2E;
   if (threadIdx.x == 0) mine[2] = 0.f;
   __syncthreads();
-  float m = fixed ? cap * LOG2E : -INFINITY, sum = 0.f;                            // exponents to base 2
+  // Exponents to base 2.  A capped logit is at least -cap, so the running maximum starts there: no value is skipped while there is none yet, and a NaN
+  // reaches the sum wherever it stands.
+  float m = fixed ? slope : -slope, sum = 0.f;
   // all of the part is requested before the first value is used, in two groups; a thread reads only what it copied itself
   const int middle = (n / 8 + 2 * CE_THREADS - 1) / (2 * CE_THREADS) * CE_THREADS * 8;
   for (int half = 0; half < 2; ++half) {
@@ -587,14 +589,10 @@ softcap_ce_cluster_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const 
     const __nv_bfloat162* h = (const __nv_bfloat162*)&raw;
 #pragma unroll
     for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(h[j]); v[2 * j] = f.x; v[2 * j + 1] = f.y; }
-    if (cap > 0.f) tanh8(raw, v, inv_cap, edge, t);
-    else {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) t[j] = v[j];
-    }
+    tanh8(raw, v, inv_cap, edge, t);
     if ((unsigned)(label - c) < 8u) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) if (c + j == label) mine[2] = cap > 0.f ? cap * t[j] : t[j];
+      for (int j = 0; j < 8; ++j) if (c + j == label) mine[2] = cap * t[j];
     }
     if (fixed) {
 #pragma unroll
@@ -604,10 +602,8 @@ softcap_ce_cluster_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const 
 #pragma unroll
       for (int j = 1; j < 8; ++j) mx = fmaxf(mx, t[j] * slope);
       if (mx > m) { sum *= exp2f(m - mx); m = mx; }
-      if (m != -INFINITY) {
 #pragma unroll
-        for (int j = 0; j < 8; ++j) sum += exp2f(fmaf(t[j], slope, -m));
-      }
+      for (int j = 0; j < 8; ++j) sum += exp2f(fmaf(t[j], slope, -m));
     }
   }
   auto merge = [](float& m, float& s, float m2, float s2) {
@@ -650,19 +646,12 @@ softcap_ce_cluster_kernel(__nv_bfloat16* __restrict__ logits, int64_t ld, const 
     const __nv_bfloat162* h = (const __nv_bfloat162*)&raw;
 #pragma unroll
     for (int j = 0; j < 4; ++j) { const float2 f = __bfloat1622float2(h[j]); v[2 * j] = f.x; v[2 * j + 1] = f.y; }
-    if (cap > 0.f) tanh8(raw, v, inv_cap, edge, t);
-    else {
+    tanh8(raw, v, inv_cap, edge, t);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) t[j] = v[j];
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float slope_of_cap = cap > 0.f ? on * fmaf(-t[j], t[j], 1.f) : on;
-      o[j] = slope_of_cap * exp2f(fmaf(t[j], slope, -lse));
-    }
+    for (int j = 0; j < 8; ++j) o[j] = on * fmaf(-t[j], t[j], 1.f) * exp2f(fmaf(t[j], slope, -lse));
     if ((unsigned)(label - c) < 8u) {
 #pragma unroll
-      for (int j = 0; j < 8; ++j) if (c + j == label) o[j] -= cap > 0.f ? on * fmaf(-t[j], t[j], 1.f) : on;
+      for (int j = 0; j < 8; ++j) if (c + j == label) o[j] -= on * fmaf(-t[j], t[j], 1.f);
     }
     st8(lr + lo + c, o);
   }
@@ -794,11 +783,16 @@ MARY_API int mary_softcap_ce(void* logits, int64_t ld, const int64_t* labels, in
                              cudaStream_t s) {
   if (rows <= 0) return MARY_OK;
   if ((V & 7) || (ld & 7)) return MARY_ERR_BAD_ARG;
-  // rows that a cluster can hold, 64 KB to a CTA (up to 128 KB with the largest cluster): read once
+  // The cluster form where there is a cap, from 8192 values on, for rows that a cluster holds at 100 KB to a CTA (two CTAs to an SM).  As few CTAs as that
+  // takes, since their meeting is what the form costs, but more while there are rows for half of the SMs only.  us, two passes / cluster of 1, 2, 4, 8,
+  // cap 30: 1024 rows of 4096 11.5 / 13.1, of 8192 22 / 18, of 50000 97 / 72, 86, 121, 202, of 151936 272 / -, -, 244, 316, of 262144 461 / 440 (8); 16 rows
+  // of 32000 11.2 / 10.2, 8.5, 6.6, 7.0.  At 128 KB one CTA fills an SM (1024 rows of 524288: 917 / 1130): only for a few rows (16: 130 / 34).
+  // Without a cap there is little arithmetic to save, and two passes are both faster (1024 rows of 262144: 292 / 327) and closer to the exact sum.
   int ctas = 1;
-  while (ctas < 8 && V > 32768 * ctas) ctas *= 2;
+  while (ctas < 8 && V > 51200 * ctas) ctas *= 2;
+  while (ctas < 8 && V >= 16384 && (int64_t)rows * ctas * 2 <= mary_num_sms() / 2) ctas *= 2;
   const int part = ((V + ctas - 1) / ctas + 7) / 8 * 8;
-  if (V >= 4096 && part <= 65536 && rows <= 65535 && ((uintptr_t)logits & 15) == 0) {
+  if (cap > 0.f && V >= 8192 && (part <= 51200 || (part <= 65536 && (int64_t)rows * ctas <= mary_num_sms())) && rows <= 65535 && ((uintptr_t)logits & 15) == 0) {
     static MarySmemSlots smem_set = {};
     if (int rc = mary_ensure_dyn_smem((const void*)softcap_ce_cluster_kernel, (size_t)part * 2, &smem_set)) return rc;
     cudaLaunchConfig_t cfg = {};
