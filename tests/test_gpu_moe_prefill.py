@@ -64,6 +64,11 @@ def test_plan_places_every_entry_once(n, k, E, nt):
     assert torch.equal(torch.zeros(E, dtype=torch.int64, device="cuda").index_add_(0, tiles[:, 0], tiles[:, 2]), counts)
 
 
+@pytest.mark.parametrize("n,k,E,nt", [(8, 8, 8, 32), (1023, 3, 16, 32), (1024, 8, 128, 32), (1032, 8, 385, 128), (4096, 1, 4096, 32), (4097, 1, 3, 128)])
+def test_plan_at_the_edges_of_a_lone_cta(n, k, E, nt):
+    test_plan_places_every_entry_once(n, k, E, nt)
+
+
 @pytest.mark.parametrize("T,E,k", [(1, 1, 1), (127, 1, 1), (129, 2, 1), (260, 3, 2), (1000, 5, 2)])
 def test_token_tiles_of_128_equal_those_of_32(T, E, k):
     """The same products through both epilogues: plain rows, and quantised for the next GEMM."""
