@@ -174,7 +174,8 @@ __global__ void mla_q_rope_kernel(const __nv_bfloat16* qb, const float* __restri
 }
 
 // The same for 8-byte aligned rows: eight lanes hold a head's 64 dims (lane j the pairs 4 j .. 4 j + 3), a warp walks QR_HEADS heads of one token, four at a
-// time, with one set of angles (4096 tokens of 64 heads: 36 us by one head per warp and 2-byte accesses).
+// time, with one set of angles (4096 tokens of 64 heads: 36 us by one head per warp and 2-byte accesses, 9.6 us so).  Up to 4096 heads in all, where every
+// warp of the form above has one and its chain is the shorter one, that form stays (3 tokens of 64 heads: 2.6 us, 3.3 us by this one; 64 of 64: 2.9 / 3.2).
 constexpr int QR_HEADS = 16;
 __global__ void __launch_bounds__(256)
 mla_q_rope_heads_kernel(const __nv_bfloat16* qb, const float* __restrict__ inv_freq, const int* __restrict__ positions, __nv_bfloat16* q_full, int H, int T,
@@ -268,7 +269,7 @@ MARY_API int mary_mla_prep(const void* qakv, int64_t ld, int q_lora, const void*
 
 static int q_rope(const void* qb, const float* inv_freq, const int* positions, void* dst, int H, int T, int64_t stride, int off, cudaStream_t s) {
   if (T <= 0) return MARY_OK;
-  if (((uintptr_t)qb | (uintptr_t)dst) % 8 == 0) {
+  if (((uintptr_t)qb | (uintptr_t)dst) % 8 == 0 && (int64_t)T * H > 4096) {
     const int64_t warps = (int64_t)T * ((H + QR_HEADS - 1) / QR_HEADS);
     MARY_LAUNCH(mla_q_rope_heads_kernel, (int)((warps + 7) / 8), 256, 0, s, (const __nv_bfloat16*)qb, inv_freq, positions, (__nv_bfloat16*)dst, H, T, stride, off);
   } else {

@@ -903,9 +903,12 @@ def mla_expand_kv(rows, w_uk_t, w_uv, H):
     ``v [N, H, 128]`` (one GEMM).  ``w_uk_t [H * 128, 512]``, ``w_uv [H * 128, 512]``."""
     N = rows.shape[0]
     k = _empty(N, H, 192, dtype=torch.bfloat16, device=rows.device)
-    check(lib().mary_gemm_bf16_grouped_columns(_p(rows), _p(w_uk_t), _p(k), N, H * 128, 512, rows.stride(0), 512, H * 192, 128, 192, _stream()),
-          "gemm_bf16_grouped_columns")
     with static_weights:
+        if N <= 64:                    # half a tile of rows: one small GEMM per head is the faster form (64 rows of 64 heads, keys and values: 16.3 / 17.9 us)
+            gemm_batched(rows, w_uk_t, k, N, 128, 512, rows.stride(0), 512, H * 192, H, 0, 128 * 512, 192)
+        else:
+            check(lib().mary_gemm_bf16_grouped_columns(_p(rows), _p(w_uk_t), _p(k), N, H * 128, 512, rows.stride(0), 512, H * 192, 128, 192, _stream()),
+                  "gemm_bf16_grouped_columns")
         v = gemm(rows[:, :512], w_uv)
     check(lib().mary_mla_fill_k_rope(_p(rows), rows.stride(0), _p(k), H, N, _stream()), "mla_fill_k_rope")
     return k, v.view(N, H, 128)

@@ -47,6 +47,12 @@ def test_query_rotation_and_shared_key_dims(H, T):
     assert K.last_status() == 0
 
 
+@pytest.mark.parametrize("T,H", [(64, 64), (65, 64), (300, 17), (4100, 1), (64, 128), (241, 17)])
+def test_query_rotation_of_many_heads(T, H):
+    """Around 4096 heads in all, from where a warp walks 16 heads: groups that are left unfilled."""
+    test_query_rotation_and_shared_key_dims(H, T)
+
+
 @pytest.mark.parametrize("q_lora", [8, 64, 1536, 1544, 6144, 6152, 36])
 def test_prep_norms_and_appends(q_lora):
     from mary_b200.ops import cuda as K
