@@ -550,7 +550,8 @@ def stream_split(units: int, span: int, sms: int = 148):
     keys: waves of CTAs x (4 us + keys of a CTA x time per key).  A lone warp needs 141 ns per key (eight keys take one chain of load, sum over the lanes,
     exponential, weighted sum), an SM gets through one key per 25 ns, and the rings let an SM hold three CTAs of 4 warps or one of 8; clusters of 4
     and 8 CTAs leave 12 and 36 SMs out.  Measured (us) for 256 units of 1024 keys of 256: 1 / 8 56, 1 / 4 57, 4 / 4 67, 2 / 4 78; for 64 units of 2000: 2 / 8
-    30, 4 / 4 33, 2 / 4 40, 1 / 8 50; for 8 of 777: 8 / 8 8, 8 / 4 9, 4 / 8 10, 1 / 4 30."""
+    30, 4 / 4 33, 2 / 4 40, 1 / 8 50; for 8 of 777: 8 / 8 8, 8 / 4 9, 4 / 8 10, 1 / 4 30.  The split is chosen as if its CTAs spread over all SMs; the estimate
+    that is returned counts what the SMs that its clusters can reach hold: 16 units of 4000 in 8 / 4 are two CTAs on some of 112 SMs, 30 us and not 22."""
     best = None
     for nsplit, usable in ((1, sms), (2, sms), (4, sms - 12), (8, sms - 36)):
         if nsplit > 1 and span < 32 * nsplit:
@@ -558,11 +559,12 @@ def stream_split(units: int, span: int, sms: int = 148):
         for warps, fit in ((4, 3), (8, 1)):
             ctas = units * nsplit
             waves = -(-ctas // max(1, fit * usable))
-            resident = min(fit, -(-ctas // sms))
-            t = waves * (4.0 + -(-span // nsplit) * max(0.141 / warps, 0.025 * resident))
-            if best is None or t < best[2]:
-                best = (nsplit, warps, t)
-    return best
+
+            def us(reach):
+                return waves * (4.0 + -(-span // nsplit) * max(0.141 / warps, 0.025 * min(fit, -(-ctas // reach))))
+            if best is None or us(sms) < best[0]:
+                best = (us(sms), nsplit, warps, us(usable))
+    return best[1:]
 
 
 def _stream_wins(q, kcache, vcache, meta, window) -> bool:
@@ -581,7 +583,7 @@ def _stream_wins(q, kcache, vcache, meta, window) -> bool:
         keys = int(np.minimum(meta.kv_lens_host, window + rq).sum() if window > 0 else meta.kv_lens_host.sum())
         span = meta.max_kv_len if window <= 0 else min(meta.max_kv_len, window + rq)
         blocks = sum(-(-n // rq) for n in meta.q_lens_host.tolist())
-        memo[key] = stream_split(blocks * Hkv, span, lib().mary_sm_count())[2] <= 10.0 + keys * Hkv * 1024 / 5.3e6
+        memo[key] = stream_split(blocks * Hkv, span, lib().mary_sm_count())[2] <= 15.0 + keys * Hkv * 1024 / 5.3e6
     return memo[key]
 
 
