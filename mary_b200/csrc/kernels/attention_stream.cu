@@ -355,24 +355,30 @@ attn_stream_kernel(const StreamParams p) {
 template <int D, int R, bool Q8, int WARPS>
 int launch(const StreamParams& p, int NB, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(p.nsplit, NB, p.Hkv);
   cfg.blockDim = dim3(WARPS * 32);
   cfg.dynamicSmemBytes = WARPS * Group<D, R, Q8>::STAGES * Group<D, R, Q8>::STAGE;
   cfg.stream = s;
   static MarySmemSlots smem_set = {};
   if (int rc = mary_ensure_dyn_smem((const void*)attn_stream_kernel<D, R, Q8, WARPS>, cfg.dynamicSmemBytes, &smem_set)) return rc;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = p.nsplit;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.nsplit;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
   // More CTAs than SMs start after their predecessor: placed while it drains they would crowd three deep onto the SMs that are free first (256 CTAs of
   // 2048 bf16 keys: 80 us instead of 66).
   cfg.numAttrs = mary_pdl_enabled() && (int64_t)p.nsplit * NB * p.Hkv <= mary_num_sms() ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, attn_stream_kernel<D, R, Q8, WARPS>, p) != cudaSuccess) return MARY_ERR_CUDA;
-  MARY_CHECK_LAUNCH();
+  // a grid has at most 65535 query blocks (as x instead, together with the splits, they took 92 -> 120 us: 8 sequences of 8000 bf16 keys, 8 kv heads)
+  for (int at = 0; at < NB; at += 65535) {
+    StreamParams part = p;
+    part.blk_seq += at;
+    part.blk_q0 += at;
+    cfg.gridDim = dim3(p.nsplit, NB - at < 65535 ? NB - at : 65535, p.Hkv);
+    if (cudaLaunchKernelEx(&cfg, attn_stream_kernel<D, R, Q8, WARPS>, part) != cudaSuccess) return MARY_ERR_CUDA;
+    MARY_CHECK_LAUNCH();
+  }
   return MARY_OK;
 }
 
@@ -399,7 +405,7 @@ MARY_API int mary_attention_stream(const void* q, const void* kc, const void* vc
                                    int RQ, int nsplit, int warps, int window, float scale, float softcap, cudaStream_t s) {
   if (NB <= 0) return MARY_OK;
   if (Hkv < 1 || Hq % Hkv || page_size < 1 || RQ < 1 || (nsplit != 1 && nsplit != 2 && nsplit != 4 && nsplit != 8) || (warps != 4 && warps != 8) ||
-      (k_sz == nullptr) != (v_sz == nullptr) || NB > 65535 || Hkv > 65535)
+      (k_sz == nullptr) != (v_sz == nullptr) || Hkv > 65535)
     return MARY_ERR_BAD_ARG;
   // rows are copied 16 bytes at a time, a lane reads D / 32 neighbouring query values at once
   const int64_t es = k_sz ? 1 : 2, qb = D / 32 * 2;

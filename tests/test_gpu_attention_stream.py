@@ -85,3 +85,26 @@ def test_stream_attention_strided_cache():
         got = K.attention_stream(q, k, vc, meta, 0.1).double()
         want = _exact(q, k.double(), vc.double(), table, [1, 1], [400, 123], 16, 0.1, 0, 0.0)
         assert (got - want).norm() / want.norm() < 2.0 ** -8
+
+
+def test_more_query_blocks_than_a_grid_has_rows():
+    """70000 sequences of one to three keys over an 8-bit cache."""
+    from mary_b200 import ops
+    from mary_b200.runtime.batch import BatchMeta
+    from mary_b200.runtime.kv_cache import Q8Pages
+    from mary_b200.ops import cuda as K
+    S = 70000
+    kv = np.arange(S, dtype=np.int32) % 3 + 1
+    meta = BatchMeta.build(np.ones(S, dtype=np.int32), kv, np.arange(S, dtype=np.int32)[:, None], 4, "cuda")
+    g = torch.Generator(device="cuda").manual_seed(4)
+    kc, vc = Q8Pages(S, 4, 1, 64, "cuda"), Q8Pages(S, 4, 1, 64, "cuda")
+    for t in (kc, vc):
+        t.codes, t.sz = Q8Pages.quantize(torch.empty(S, 4, 1, 64, device="cuda").normal_(0, 1, generator=g))
+    q = torch.empty(S, 1, 64, dtype=torch.bfloat16, device="cuda").normal_(0, 0.3, generator=g)
+    got = ops.paged_attention(q, kc, vc, meta, 0.5)
+    k64, v64 = ((t.codes.double() * t.sz[..., :1].double() + t.sz[..., 1:].double())[:, :, 0] for t in (kc, vc))
+    x = torch.einsum("sd,std->st", q[:, 0].double(), k64) * 0.5
+    x = x.masked_fill(torch.arange(4, device="cuda")[None] >= torch.from_numpy(kv).cuda()[:, None], -torch.inf)
+    want = torch.einsum("st,std->sd", torch.softmax(x, -1), v64)
+    assert (got[:, 0].double() - want).norm() / want.norm() < 2.0 ** -8
+    assert K.last_status() == 0
