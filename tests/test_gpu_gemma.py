@@ -65,3 +65,15 @@ def test_gpu_generation_batching_invariance():
     together = _engine(gpu, "cuda", torch.bfloat16).generate(prompts, 8)
     # identical kernels and reduction orders per row -> identical tokens
     assert together == alone
+
+
+def test_logits_of_rows_with_any_stride():
+    """Hidden rows that are a transposed view: the head takes them as the bf16 product did."""
+    cfg = Gemma4TextConfig(hidden_size=256, num_hidden_layers=1, num_attention_heads=4, num_key_value_heads=1, head_dim=64, intermediate_size=512, vocab_size=1024,
+                           sliding_window=16)
+    model = Gemma4Model(cfg, dtype=torch.bfloat16, device="cuda")
+    init_random_(model, 0)
+    x = torch.randn(256, 5, device="cuda").bfloat16().t()
+    assert x.stride(1) != 1
+    with torch.no_grad():
+        assert torch.equal(model.logits(x), model.logits(x.contiguous()))
