@@ -8,7 +8,7 @@
 //     q . (s c + z) = s (q . c) + z sum(q), and sum_j p_j (s_j c_j + z_j) = sum_j (p_j s_j) c_j + sum_j p_j z_j;
 //   * the dot products of a group of keys are completed by a halving exchange that leaves ONE (key, row) total in each lane; scale, mask, maximum,
 //     exponential and sum then run once per (key, row), in parallel over the lanes, and only the weights are broadcast;
-//   * every warp has a ring of groups of its own in shared memory, filled by asynchronous copies a few groups ahead (what is in flight does not live in
+//   * every warp has a ring of groups of its own in shared memory, filled by asynchronous copies at least one group ahead (what is in flight does not live in
 //     registers, and no warp waits for another).
 //
 // The key range of a (query block, kv head) is cut between the CTAs of a cluster, which merge their partial results through distributed shared
@@ -111,7 +111,9 @@ __device__ __forceinline__ void copy_async8(uint32_t dst, const void* src) {
 }
 
 constexpr int STREAM_GROUP = 8192;           // K and V bytes of a group at most
-constexpr int STREAM_RING = 16384;            // bytes of a warp's ring: two groups of bf16 rows, four of codes (three groups: 120 us instead of 104, fewer CTAs fit)
+// Bytes of a warp's ring, but two groups at least: two of bf16 rows or of codes of 256 with their scales (16896 bytes), three to eight of smaller ones.  Three
+// groups of bf16 rows: 120 us instead of 104, fewer CTAs fit.
+constexpr int STREAM_RING = 16384;
 template <int D, int R, bool Q8> struct Group {
   static constexpr int ROW = D * (Q8 ? 1 : 2);                         // bytes of a key or value row
   static constexpr int FIT = STREAM_GROUP / (2 * ROW);

@@ -539,7 +539,7 @@ static int gemm_impl(const void* X, const void* W, void* out, int M, int N, int 
   if (split_k < 1) split_k = 1;
   const bool sk_epi = epi == EPI_SK_BF16 || epi == EPI_SK_F32;
   if (split_k > 1 && epi != EPI_RED_F32 && !sk_epi) return MARY_ERR_BAD_ARG;
-  if (sk_epi && (glu || !ws || !counters)) return MARY_ERR_BAD_ARG;
+  if (sk_epi && glu) return MARY_ERR_BAD_ARG;
   if (glu && epi == EPI_RED_F32) return MARY_ERR_BAD_ARG;
   // The two-SM kernel (gemm_pair.cu) takes plain products of more rows than one 128-row tile, with the GLU in its epilogue, and, with the weights
   // as the row operand, the products of fewer rows whose K is to be cut so that every SM works: 15.5 against 18.0 us at 1 x 8192 x 3840, 24.2
@@ -556,6 +556,7 @@ static int gemm_impl(const void* X, const void* W, void* out, int M, int N, int 
     if (!mary_gemm_pair_plan(N, M, K, false, (M + 31) / 32 * 32, &plan)) return MARY_ERR_BAD_ARG;
     return mary_gemm_pair_run(W, X, N, M, K, ldw, ldx, true, o, plan, stream);
   }
+  if (sk_epi && (!ws || !counters)) return MARY_ERR_BAD_ARG;
   const bool use_swap = glu ? true : (swap < 0 ? (M <= 256) : swap != 0);
   // GLU without swap would need the weight operand on the column side, so here GLU implies swap.
   GemmParams p;
@@ -706,12 +707,12 @@ MARY_API int mary_gemm_bf16(const void* X, const void* W, void* out, int M, int 
                    0, false, nullptr, nullptr, 0, 0, glu_limit);
 }
 
-// out = act(X W^T) on the first un_cols output features (act: 1 tanh-form GELU, 2 SiLU), X W^T on the others; bf16.  ws null: no split of K, else
-// stream-K as mary_gemm_bf16_splitk with split_k = 0.
+// out = act(X W^T) on the first un_cols output features (act: 1 tanh-form GELU, 2 SiLU), X W^T on the others; bf16.  cut: K is cut so
+// that every SM works, as by mary_gemm_bf16_splitk with split_k = 0.
 MARY_API int mary_gemm_bf16_act(const void* X, const void* W, void* out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo, int act, int un_cols,
-                                float* ws, int64_t ws_floats, int* counters, int n_counters, cudaStream_t stream) {
-  return gemm_impl(X, W, out, M, N, K, ldx, ldw, ldo, 1, 0, 0, 0, nullptr, 1.0f, 0, ws ? EPI_SK_BF16 : EPI_STORE_BF16, 1, -1, nullptr, 0, 0, 0, stream,
-                   ws, ws_floats, counters, n_counters, ws != nullptr, nullptr, nullptr, 0, 0, 0.f, act, un_cols);
+                                int cut, cudaStream_t stream) {
+  return gemm_impl(X, W, out, M, N, K, ldx, ldw, ldo, 1, 0, 0, 0, nullptr, 1.0f, 0, cut ? EPI_SK_BF16 : EPI_STORE_BF16, 1, -1, nullptr, 0, 0, 0, stream,
+                   nullptr, 0, nullptr, 0, cut != 0, nullptr, nullptr, 0, 0, 0.f, act, un_cols);
 }
 
 // Grouped (mixture-of-experts) GEMM with unquantised expert weights: out[rows_pad, N] = X[rows_pad, K] * W[expert of the row's tile]^T,
@@ -735,7 +736,8 @@ MARY_API int mary_gemm_bf16_grouped(const void* X, const void* W, void* out, int
 MARY_API int mary_gemm_bf16_splitk(const void* X, const void* W, void* out, int M, int N, int K, int64_t ldx, int64_t ldw, int64_t ldo,
                                    const float* bias, float alpha, int out_f32, int split_k, int swap, float* ws, int64_t ws_floats,
                                    int* counters, int n_counters, cudaStream_t stream) {
-  // split_k == 0: stream-K (equal runs of K-blocks per CTA)
+  // split_k == 0, swap < 0: the two-SM kernel, which cuts K inside a cluster and needs no scratch.  split_k == 0 with an order asked for: stream-K (equal runs
+  // of K-blocks per CTA), whose sums are added in the order of arrival
   return gemm_impl(X, W, out, M, N, K, ldx, ldw, ldo, 1, 0, 0, 0, bias, alpha, 0, out_f32 ? EPI_SK_F32 : EPI_SK_BF16,
                    split_k == 0 ? 1 : split_k, swap, nullptr, 0, 0, 0, stream, ws, ws_floats, counters, n_counters, split_k == 0);
 }

@@ -105,7 +105,7 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint16_t mask) {
                ::"r"(smem_u32(bar)), "h"(mask) : "memory");
 }
 
-// tiles of this cluster, in bands of `raster` column tiles (row tiles fastest inside a band) so that the clusters that run together
+// tiles of this cluster, in bands of `raster` column tiles (rows of a band one after the other, its columns fastest) so that the clusters that run together
 // cover a compact block of the output
 __device__ __forceinline__ void tile_at(const PairParams& p, int t, int& tr, int& tc) {
   if (p.raster > 0) {

@@ -242,8 +242,8 @@ def determinism(mutate: bool) -> list[str]:
     """Run-to-run stability (golden/determinism/cmp.py, nanscan.py): the same decode steps from the same state, twice — emitted
     tokens and logits must be bit-identical and free of NaN / Inf.  The reference traced its own flips (43 of 503 positions) to the
     GPU reading reclaimed file pages; here weights live in device memory, so any flip is a kernel's.  On a GPU the check runs the
-    MoE decoder's step (stream-K GEMMs included: their partial sums are added in arrival order, so the LOGITS may differ in the
-    last bit; the gate reports that separately and fails only on a token flip or a non-finite value)."""
+    MoE decoder's step (where a kernel adds partial sums in the order of their arrival the LOGITS may differ in the last bit; the gate
+    reports that separately and fails only on a token flip or a non-finite value)."""
     from .models.moe import MoEDecoder, init_random_, tiny_moe_config
     from .runtime.batch import BatchMeta
     from .runtime.kv_cache import PagedKVCache

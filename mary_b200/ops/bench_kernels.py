@@ -64,7 +64,7 @@ def bench_gemm(shapes=None):
         fl = 2.0 * M * N * Kd / ours / 1e9
         gb = (M * Kd + N * Kd + M * N) * 2 / ours / 1e6
         frac = max(fl / tf, gb / hbm)
-        print(f"{M:>6} {N:>6} {Kd:>6} {ours:>9.4f} {th:>9.4f} {fl:>8.1f} {gb:>7.0f}  {frac:.2f} ({"stream-K" if sk > 1 else "whole tiles"})")
+        print(f"{M:>6} {N:>6} {Kd:>6} {ours:>9.4f} {th:>9.4f} {fl:>8.1f} {gb:>7.0f}  {frac:.2f} ({"K cut" if sk > 1 else "whole tiles"})")
     assert K.last_status() == 0
 
 
@@ -257,8 +257,8 @@ def bench_floor(reps: int = 200):
     x = torch.randn(48, 7168, device="cuda").bfloat16()
     cases = {
         "gemm 48x128x512 (one tile)": (lambda a=torch.randn(48, 512, device="cuda").bfloat16(), w=torch.randn(128, 512, device="cuda").bfloat16(): K.gemm(a, w)),
-        "gemm 48x2112x7168 (stream-K)": (lambda w=(torch.randn(2112, 7168, device="cuda") * 0.02).bfloat16(): K.linear(x, w)),
-        "gemm 48x7168x8192 (stream-K)": (lambda a=torch.randn(48, 8192, device="cuda").bfloat16(), w=(torch.randn(7168, 8192, device="cuda") * 0.02).bfloat16(): K.linear(a, w)),
+        "gemm 48x2112x7168 (K cut)": (lambda w=(torch.randn(2112, 7168, device="cuda") * 0.02).bfloat16(): K.linear(x, w)),
+        "gemm 48x7168x8192 (K cut)": (lambda a=torch.randn(48, 8192, device="cuda").bfloat16(), w=(torch.randn(7168, 8192, device="cuda") * 0.02).bfloat16(): K.linear(a, w)),
         "gemm 48x384x7168 f32 (router)": (lambda w=(torch.randn(384, 7168, device="cuda") * 0.02).bfloat16(): K.linear_f32(x, w)),
         "rmsnorm 48x7168": (lambda g=torch.ones(7168, device="cuda").bfloat16(): K.rmsnorm(x, g)),
         # one token: the tensor-core GEMM against the matrix-vector stage of the fused layer step (weights L2-resident: the floor)

@@ -141,7 +141,8 @@ def gemm(x, w, out=None, bias=None, alpha: float = 1.0, glu: str | None = None, 
 
 
 def _auto_split_k(M: int, N: int, K: int) -> int:
-    """GEMMs with few output tiles cannot fill 148 SMs; split K until they do (mirrors the launcher's tile choice)."""
+    """Into how many parts K would be cut for the one-SM kernel's tiles to fill 148 SMs; 1: not at all.  Above 1 the product goes to the two-SM kernel
+    whatever its rows, which then decides by itself how to cut; at 1 products of at most 128 rows stay on the one-SM kernel."""
     if M <= 256:
         bn = 32 if M <= 32 else 64 if M <= 64 else 128 if M <= 128 else 256
         tiles = ((N + 127) // 128) * ((M + bn - 1) // bn)
@@ -151,8 +152,8 @@ def _auto_split_k(M: int, N: int, K: int) -> int:
         while bn > 64 and tr * ((N + bn - 1) // bn) < 148:
             bn //= 2
         tiles = tr * ((N + bn - 1) // bn)
-    # measured on a B200 at 48 and 384 rows: from ~90 tiles on, and for short K (a tile's main loop is then a few stages long and
-    # the partial-tile traffic of a split outweighs the idle SMs), the unsplit kernel is the faster one
+    # measured at 48 and 384 rows on the one-SM kernel alone: from ~90 tiles on, and for short K (a tile's main loop is then a few stages long and the
+    # partial-tile traffic of a split outweighs the idle SMs), the unsplit kernel is the faster one
     if tiles >= 90 or K <= 2048:
         return 1
     return max(1, min(K // 512, (148 + tiles - 1) // tiles))
@@ -173,13 +174,15 @@ def gemm_pair(x, w, bn: int, splits: int = 1, swap: bool = False, glu: str | Non
     check(lib().mary_gemm_bf16_pair(_p(x), _p(w), _p(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), g, int(f32), bn, splits, int(swap),
                                     _stream()), "gemm_bf16_pair")
     return out
+
+
 _SK_WS: dict = {}
 SK_WS_FLOATS = 4 << 20          # 16 MiB of accumulator tiles
 SK_COUNTERS = 8192
 
 
 def _sk_workspace(dev):
-    """Scratch of the split-K GEMM (f32 accumulator tiles + per-tile arrival counters, zero between calls), one per device;
+    """Scratch of the one-SM split-K GEMM (f32 accumulator tiles + per-tile arrival counters, zero between calls), one per device;
     calls on one stream share it.  Created on first use — before any stream capture, since warm-up steps run eagerly first."""
     key = dev.index if dev.index is not None else torch.cuda.current_device()
     if key not in _SK_WS:
@@ -189,20 +192,21 @@ def _sk_workspace(dev):
 
 def gemm_splitk(x, w, split_k: int, out=None, f32: bool = False, bias=None, swap: int = -1, alpha: float = 1.0):
     """``x @ w^T`` with K cut into ``split_k`` slices reduced inside the kernel (every slice adds into an f32 accumulator tile in
-    scratch; the slice that finishes last converts and stores it and leaves the scratch zero): no zero-fill, no cast pass.  ``split_k=0`` is stream-K: the K-blocks of all tiles are dealt out in
-    equal contiguous runs, one per SM, so every SM streams the same share of the weights whatever the tile count.  Falls back
-    to the atomic path when the shape outgrows the scratch."""
+    scratch; the slice that finishes last converts and stores it and leaves the scratch zero): no zero-fill, no cast pass.  ``split_k=0`` leaves the cut to
+    the two-SM kernel (``csrc/kernels/gemm_pair.cu``: between the pairs of a cluster, no scratch, the same bits in every run); with an operand order asked
+    for (``swap`` 0 or 1) it is stream-K, the K-blocks of all tiles dealt out in equal contiguous runs, one per SM.  Falls back to the atomic path when the
+    shape outgrows the scratch."""
     _bf16(x), _bf16(w)
     if bias is not None and bias.dtype != torch.float32:
         bias = bias.float()
     M, K = x.shape
     N = w.shape[0]
-    ws, cnt = _sk_workspace(x.device)
+    ws, cnt = (None, None) if split_k == 0 and swap < 0 else _sk_workspace(x.device)
     if out is None:
         out = _empty(M, N, dtype=torch.float32 if f32 else torch.bfloat16, device=x.device)
     rc = lib().mary_gemm_bf16_splitk(_p(x), _p(w), _p(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), _p(bias), alpha, int(f32),
-                                     split_k, swap, _p(ws), ws.numel(), _p(cnt), cnt.numel(), _stream())
-    if rc == 4:                                             # scratch too small for this shape
+                                     split_k, swap, _p(ws), 0 if ws is None else ws.numel(), _p(cnt), 0 if cnt is None else cnt.numel(), _stream())
+    if rc == 4 and ws is not None:                          # scratch too small for this shape
         red = gemm(x, w, alpha=alpha, epi="red", split_k=split_k or _auto_split_k(M, N, K))
         if bias is not None:
             red += bias
@@ -304,7 +308,7 @@ def linear_f32(x, w, split_k: int | None = None, alpha: float = 1.0):
         return gemm_splitk(x, w, 0 if split_k is None else sk, f32=True, alpha=alpha) if sk > 1 else gemm(x, w, alpha=alpha, epi="f32")
 
 
-declare("mary_gemm_bf16_act", "pppiiilllii" + "plpis")
+declare("mary_gemm_bf16_act", "pppiiilllii" + "is")
 
 
 def linear_act(x, w, act: str, cols: int):
@@ -318,16 +322,9 @@ def linear_act(x, w, act: str, cols: int):
         return step_matvec(x, w, mode=act, act_rows=cols)
     out = _empty(M, N, dtype=torch.bfloat16, device=x.device)
     code = {"gelu": 1, "silu": 2}[act]
-    ws = cnt = None
-    if _auto_split_k(M, N, K) > 1:
-        ws, cnt = _sk_workspace(x.device)
-    sk = (None, 0, None, 0) if ws is None else (_p(ws), ws.numel(), _p(cnt), cnt.numel())
-    args = lambda *sk: (_p(x), _p(w), _p(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), code, cols, *sk, _stream())  # noqa: E731
     with static_weights:
-        rc = lib().mary_gemm_bf16_act(*args(*sk))
-        if rc != 0 and ws is not None:             # more tiles than the scratch holds: without the split
-            rc = lib().mary_gemm_bf16_act(*args(None, 0, None, 0))
-    check(rc, "gemm_bf16_act")
+        check(lib().mary_gemm_bf16_act(_p(x), _p(w), _p(out), M, N, K, x.stride(0), w.stride(0), out.stride(0), code, cols, int(_auto_split_k(M, N, K) > 1),
+                                       _stream()), "gemm_bf16_act")
     return out
 
 
