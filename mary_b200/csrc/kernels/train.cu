@@ -508,7 +508,7 @@ __global__ void __launch_bounds__(1024) softcap_ce_kernel(__nv_bfloat16* __restr
 }
 
 // The same for a cap > 0, with the row kept in shared memory by a cluster, whose CTAs hold neighbouring parts of it: the logits are read once and written
-// once, and two or three CTAs of an SM overlap their loads, arithmetic and stores.  A value costs one exponential per pass: tanh is its series x (1 - x^2 / 3 + ..) to
+// once, and two CTAs of an SM overlap their loads, arithmetic and stores.  A value costs one exponential per pass: tanh is its series x (1 - x^2 / 3 + ..) to
 // x^13 (relative error below 1e-8 up to 0.35) in packed pairs, the exponential form only for vectors with a larger argument; and with 0 < cap <= 40 the
 // cap itself is the reference of the sum, which needs no running maximum (exp(-2 cap) stays a normal number).  The form above reads the row twice from
 // memory and takes six special-function results per value: 533 us for 1024 rows of 262144, this form 437 us.
